@@ -312,7 +312,7 @@ int ensure_krylov(cg_ctx *c, int m, int maxit, size_t elem_bytes, int extra = 0)
         CG_CU(cudaMalloc((void **)&c->kp.gpart, sizeof(double) * std::max(4 * ng2 * (size_t)dots2_part_ld(mc),
                                                                           ngs * (size_t)sstep_part_ld(mc))));
         CG_CU(cudaMalloc((void **)&c->kp.tickets, sizeof(unsigned int) * ngroups));
-        CG_CU(cudaMemset(c->kp.tickets, 0, sizeof(unsigned int) * ngroups));
+        CG_CU(cudaMemsetAsync(c->kp.tickets, 0, sizeof(unsigned int) * ngroups, c->stream));
         CG_CU(cudaMalloc((void **)&c->kp.ss, sizeof(double2) * (size_t)sstep_scratch_elems(mc)));
         CG_CU(cudaMalloc((void **)&c->kp.npart, sizeof(double) * np));
         CG_CU(cudaMalloc((void **)&c->kp.Hm, sizeof(double2) * (size_t)(mc + 1) * (mc + 1)));
@@ -787,7 +787,7 @@ int cugmres_create(cg_ctx **out, int device) {
         cugmres_destroy(c);
         return CG_ERR_CUDA;
     }
-    cudaMemset(c->st, 0, sizeof(DevState));
+    cudaMemsetAsync(c->st, 0, sizeof(DevState), c->stream);
     *out = c;
     return CG_OK;
 }

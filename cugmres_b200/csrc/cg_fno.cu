@@ -1140,8 +1140,9 @@ int ensure_twiddles(cg_fno *f, int H, int W) {
     for (int m = 0; m < W; m++) tw[m] = make_float2((float)cos(2 * pi * m / W), (float)sin(2 * pi * m / W));
     FN_CU(cudaMalloc(&f->twh, sizeof(float2) * H));
     FN_CU(cudaMalloc(&f->tww, sizeof(float2) * W));
-    FN_CU(cudaMemcpy(f->twh, th.data(), sizeof(float2) * H, cudaMemcpyHostToDevice));
-    FN_CU(cudaMemcpy(f->tww, tw.data(), sizeof(float2) * W, cudaMemcpyHostToDevice));
+    FN_CU(cudaMemcpyAsync(f->twh, th.data(), sizeof(float2) * H, cudaMemcpyHostToDevice, f->stream));
+    FN_CU(cudaMemcpyAsync(f->tww, tw.data(), sizeof(float2) * W, cudaMemcpyHostToDevice, f->stream));
+    FN_CU(cudaStreamSynchronize(f->stream));  // applications inside a solve read them on the solver's stream
     f->tw_H = H;
     f->tw_W = W;
     return CG_OK;
@@ -1394,7 +1395,8 @@ int prepare(cg_fno *net, int N, float k0h) {
     if (!net) return CG_ERR_INVALID;
     std::lock_guard<std::mutex> lk(net->mu);
     FN_TRY(prepare_grid(net, 1, N, N));
-    FN_CU(cudaMemcpy(net->k0h, &k0h, sizeof(float), cudaMemcpyHostToDevice));
+    FN_CU(cudaMemcpyAsync(net->k0h, &k0h, sizeof(float), cudaMemcpyHostToDevice, net->stream));
+    FN_CU(cudaStreamSynchronize(net->stream));  // the solve's stream reads it
     net->apply_k0h = k0h;
     return CG_OK;
 }
@@ -1521,11 +1523,13 @@ extern "C" int cugmres_fno_set_params(cg_fno *f, const float *params) {
     if (!f || !params) return CG_ERR_INVALID;
     std::lock_guard<std::mutex> lk(f->mu);
     FN_CU(cudaSetDevice(f->device));
-    FN_CU(cudaStreamSynchronize(f->stream));
-    FN_CU(cudaMemcpy(f->p, params, sizeof(float) * NPARAM, cudaMemcpyHostToDevice));
-    FN_CU(cudaMemset(f->m, 0, sizeof(float) * NPARAM));
-    FN_CU(cudaMemset(f->v, 0, sizeof(float) * NPARAM));
-    FN_CU(cudaMemset(f->err, 0, sizeof(int)));
+    // On the network's own (non-blocking) stream: a copy on the default stream may
+    // still be on its way from the driver's staging buffer when cudaMemcpy returns,
+    // and the packing kernel below would read the old parameters.
+    FN_CU(cudaMemcpyAsync(f->p, params, sizeof(float) * NPARAM, cudaMemcpyHostToDevice, f->stream));
+    FN_CU(cudaMemsetAsync(f->m, 0, sizeof(float) * NPARAM, f->stream));
+    FN_CU(cudaMemsetAsync(f->v, 0, sizeof(float) * NPARAM, f->stream));
+    FN_CU(cudaMemsetAsync(f->err, 0, sizeof(int), f->stream));
     f->step = 0;
     f->fwd_B = 0;
     FN_TRY(pack_weights(f, f->stream));

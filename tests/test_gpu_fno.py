@@ -270,3 +270,19 @@ def test_fgmres_mixed_precision_learned(trained_res, solver):
                            preconditioner="learned", learned_x0=True)
     solver.set_preconditioner(None)
     assert info["status"] == 0 and info["rel_residual_true"] <= 1e-10
+
+
+def test_fno_set_params_is_complete_on_return(cuda_device):
+    """The BF16 copies that set_params makes for the tensor cores come from the
+    new parameters: a network loaded once gives bitwise the gradient of one
+    loaded twice (the copy of the vector had been able to arrive after them)."""
+    p = _params(3)
+    chi, k0h, r, x = _inputs(2, 32, 32, 4)
+    for _ in range(8):
+        net = learned.FNO(device=0, seed=0)
+        net.set_params(p)
+        once = net.loss_grad(chi, k0h, r, x)
+        net.set_params(p)
+        twice = net.loss_grad(chi, k0h, r, x)
+        net.close()
+        assert once[0] == twice[0] and np.array_equal(once[1], twice[1])
