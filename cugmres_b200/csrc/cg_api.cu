@@ -82,8 +82,13 @@ struct cg_ctx {
     // the next block's Newton chain (fork and join events)
     cudaStream_t side_stream = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-    cudaGraphExec_t gexec = nullptr;
-    unsigned char gkey[256] = {0};
+    // two slots: a design loop alternates solves with A and with A^T
+    struct CycleGraph {
+        cudaGraphExec_t exec = nullptr;
+        unsigned char key[256] = {0};
+        unsigned long long used = 0;
+    } graphs[2];
+    unsigned long long graph_clock = 0;
     // learned preconditioner (flexible GMRES)
     cg_fno *net = nullptr;
     double k0h = 0.0;
@@ -241,8 +246,10 @@ void free_operator(cg_ctx *c) {
 }
 
 void free_graph(cg_ctx *c) {
-    if (c->gexec) cudaGraphExecDestroy(c->gexec);
-    c->gexec = nullptr;
+    for (auto &g : c->graphs) {
+        if (g.exec) cudaGraphExecDestroy(g.exec);
+        g.exec = nullptr;
+    }
 }
 
 void free_krylov(cg_ctx *c) {
@@ -1110,16 +1117,13 @@ int cugmres_solve(cg_ctx *c, const cg_c128 *b, cg_c128 *x, const cg_opts *opts_i
     const bool bd = is_device_ptr(b), xd = is_device_ptr(x);
     if (!bd && !all_finite((const double *)b, 2 * (size_t)n)) return CG_ERR_NONFINITE;
     if (!xd && !o.zero_x0 && !all_finite((const double *)x, 2 * (size_t)n)) return CG_ERR_NONFINITE;
-    const double2 *bp = (const double2 *)b;
-    double2 *xp = (double2 *)x;
-    if (!bd) {
-        CG_CU(cudaMemcpyAsync(c->bbuf, b, bytes, cudaMemcpyHostToDevice, s));
-        bp = c->bbuf;
-    }
-    if (!xd) {
-        xp = c->xbuf;
-        if (!o.zero_x0) CG_CU(cudaMemcpyAsync(xp, x, bytes, cudaMemcpyHostToDevice, s));
-    }
+    // The solve works on the context's own copies of b and x, so that the cycle's
+    // graph does not depend on where the caller's vectors lie (a new right-hand
+    // side had the cycle captured again); the shift run below is handed them.
+    const double2 *bp = c->bbuf;
+    double2 *xp = c->in_probe ? (double2 *)x : c->xbuf;
+    if (b != (const cg_c128 *)c->bbuf) CG_CU(cudaMemcpyAsync(c->bbuf, b, bytes, cudaMemcpyDefault, s));
+    if (!o.zero_x0) CG_CU(cudaMemcpyAsync(xp, x, bytes, cudaMemcpyDefault, s));
     if (o.zero_x0) CG_CU(cudaMemsetAsync(xp, 0, bytes, s));
 
     // s-step: the Newton shifts are the Leja-ordered Ritz values of a short
@@ -1245,7 +1249,7 @@ int cugmres_solve(cg_ctx *c, const cg_c128 *b, cg_c128 *x, const cg_opts *opts_i
     // One restart cycle: `steps` Arnoldi steps (launches after the device
     // stops the cycle return at once), back-solve and solution update.
     bool use_prec = learned;  // this cycle runs the learned preconditioner
-    auto enqueue_cycle = [&](int steps, cudaStream_t q) -> int {
+    auto enqueue_steps = [&](int steps, cudaStream_t q) -> int {
         for (int i = 0; i < steps; i++) {
             if (delayed) {
                 // w = A u_k into V[k+1]; one dot pass; normalisation + Givens; one axpy pass
@@ -1283,11 +1287,18 @@ int cugmres_solve(cg_ctx *c, const cg_c128 *b, cg_c128 *x, const cg_opts *opts_i
             CG_LAUNCH(launch_givens(kp, q));
             CG_TRY(prof_mark(c, cp, CG_PHASE_SMALL, i, q));
         }
+        return CG_OK;
+    };
+    auto enqueue_update = [&](cudaStream_t q) -> int {
         CG_LAUNCH(launch_backsolve(kp, q));
         CG_TRY(prof_mark(c, cp, CG_PHASE_SMALL, -1, q));
         CG_LAUNCH(launch_axpy(prec, 0, use_prec ? c->Z : c->V, n, kp, kp.y, 1.0, NJ_NCOL, xs, 0, 1, nax, GATE_NONE, q));
         CG_TRY(prof_mark(c, cp, CG_PHASE_UPDATE, -1, q));
         return CG_OK;
+    };
+    auto enqueue_cycle = [&](int steps, cudaStream_t q) -> int {
+        CG_TRY(enqueue_steps(steps, q));
+        return enqueue_update(q);
     };
     // s-step cycles: ceil(m / S) blocks of
     // S shifted matvecs, two block Gram-Schmidt passes and the Hessenberg /
@@ -1437,30 +1448,45 @@ int cugmres_solve(cg_ctx *c, const cg_c128 *b, cg_c128 *x, const cg_opts *opts_i
     };
     auto launch_cycle_graph = [&]() -> int {
         make_key();
-        if (!c->gexec || memcmp(c->gkey, key, sizeof(key)) != 0) {
-            free_graph(c);
+        cg_ctx::CycleGraph *slot = nullptr;
+        for (auto &g : c->graphs)
+            if (g.exec && memcmp(g.key, key, sizeof(key)) == 0) slot = &g;
+        if (!slot) {
+            slot = c->graphs[0].used <= c->graphs[1].used ? &c->graphs[0] : &c->graphs[1];
+            if (slot->exec) cudaGraphExecDestroy(slot->exec);
+            slot->exec = nullptr;
             if (!c->cap_stream) CG_CU(cudaStreamCreateWithFlags(&c->cap_stream, cudaStreamNonBlocking));
-            cudaGraph_t g = nullptr;
-            CG_CU(cudaStreamBeginCapture(c->cap_stream, cudaStreamCaptureModeThreadLocal));
-            int e1 = ss_on ? enqueue_cycle_ss(c->cap_stream, 0, ss_nblk, true)
-                           : enqueue_cycle(m + (delayed ? 1 : 0), c->cap_stream);
-            int e2 = e1 == CG_OK ? enqueue_begin(c->cap_stream) : e1;
-            cudaError_t ce = cudaStreamEndCapture(c->cap_stream, &g);
-            if (e2 != CG_OK || ce != cudaSuccess) {
-                if (g) cudaGraphDestroy(g);
-                cudaGetLastError();
-                return e2 != CG_OK ? e2 : CG_ERR_CUDA;
+            if (!ss_on) {
+                CG_TRY(cycle_graph(
+                    kp, c->cap_stream, [&](cudaStream_t q) { return enqueue_steps(LOOP_STEPS, q); },
+                    [&](cudaStream_t q) -> int {
+                        CG_TRY(enqueue_update(q));
+                        return enqueue_begin(q);
+                    },
+                    &slot->exec));
+            } else {
+                cudaGraph_t g = nullptr;
+                CG_CU(cudaStreamBeginCapture(c->cap_stream, cudaStreamCaptureModeThreadLocal));
+                int e1 = enqueue_cycle_ss(c->cap_stream, 0, ss_nblk, true);
+                int e2 = e1 == CG_OK ? enqueue_begin(c->cap_stream) : e1;
+                cudaError_t ce = cudaStreamEndCapture(c->cap_stream, &g);
+                if (e2 != CG_OK || ce != cudaSuccess) {
+                    if (g) cudaGraphDestroy(g);
+                    cudaGetLastError();
+                    return e2 != CG_OK ? e2 : CG_ERR_CUDA;
+                }
+                ce = cudaGraphInstantiate(&slot->exec, g, 0);
+                cudaGraphDestroy(g);
+                if (ce != cudaSuccess) {
+                    slot->exec = nullptr;
+                    cudaGetLastError();
+                    return CG_ERR_CUDA;
+                }
             }
-            ce = cudaGraphInstantiate(&c->gexec, g, 0);
-            cudaGraphDestroy(g);
-            if (ce != cudaSuccess) {
-                c->gexec = nullptr;
-                cudaGetLastError();
-                return CG_ERR_CUDA;
-            }
-            memcpy(c->gkey, key, sizeof(key));
+            memcpy(slot->key, key, sizeof(key));
         }
-        CG_CU(cudaGraphLaunch(c->gexec, s));
+        slot->used = ++c->graph_clock;
+        CG_CU(cudaGraphLaunch(slot->exec, s));
         return CG_OK;
     };
 
@@ -1605,7 +1631,7 @@ int cugmres_solve(cg_ctx *c, const cg_c128 *b, cg_c128 *x, const cg_opts *opts_i
         const int nh = std::min(res_hist_len, hs.it + 1);
         CG_CU(cudaMemcpyAsync(res_hist, kp.hist, sizeof(double) * nh, cudaMemcpyDeviceToHost, s));
     }
-    if (!xd) CG_CU(cudaMemcpyAsync(x, xp, bytes, cudaMemcpyDeviceToHost, s));
+    if (!c->in_probe) CG_CU(cudaMemcpyAsync(x, xp, bytes, cudaMemcpyDefault, s));
     CG_CU(cudaStreamSynchronize(s));
     if (result) {
         result->status = status;

@@ -96,8 +96,8 @@ extern "C" int cugmres_solve_batch(int device, int nsys, const cg_system *sys, c
 // every kernel of an Arnoldi step is ONE launch for the whole bucket, the
 // system being blockIdx.y (KrylovPtrs::sys_ws / sys_v, MatvecArgs::sys_*).
 // A system that stops (converged, budget, breakdown) returns at once from
-// every later launch of its bucket; the restart cycle (restart + 1 delayed
-// CGS2 steps, back-solve, update, the next true residual and cycle decisions
+// every later launch of its bucket; the restart cycle (delayed CGS2 steps while
+// a system runs, back-solve, update, the next true residual and cycle decisions
 // of all systems) is captured once per bucket as a CUDA graph and replayed
 // with one launch per cycle, one host synchronisation per cycle.
 // Scope: FP64 or mixed precision (complex64 cycles, FP64 residual and
@@ -374,8 +374,8 @@ int solve_bucket(cg_ctx *ctx, const cg_system *sys, const std::vector<int> &idx,
         BK_LAUNCH(launch_cycle_begin(kp, nrb, q));
         return CG_OK;
     };
-    auto enqueue_cycle = [&](cudaStream_t q) -> int {
-        for (int i = 0; i < m + 1; i++) {
+    auto enqueue_steps = [&](cudaStream_t q) -> int {
+        for (int i = 0; i < LOOP_STEPS; i++) {
             BK_LAUNCH(launch_rows_forward(prec, ap, vk, nullptr, kp.st, GATE_STOP, q));
             BK_LAUNCH(launch_cols_convolve(prec, ap, kp.st, GATE_STOP, q));
             BK_LAUNCH(launch_rows_inverse(prec, 0, prec, ap, vk, nullptr, nullptr, vk1, nullptr, kp.st, GATE_STOP, q));
@@ -383,31 +383,17 @@ int solve_bucket(cg_ctx *ctx, const cg_system *sys, const std::vector<int> &idx,
             BK_LAUNCH(launch_dcgs2_step(kp, q));
             BK_LAUNCH(launch_axpy2(prec, bb.V, n, kp, nax2, sms_eff, q));
         }
-        BK_LAUNCH(launch_backsolve(kp, q));
-        BK_LAUNCH(launch_axpy(prec, 0, bb.V, n, kp, kp.y, 1.0, NJ_NCOL, xs, 0, 1, nax, GATE_NONE, q));
         return CG_OK;
     };
-    // capture [cycle + next residual and decisions] once; replay per cycle
+    auto enqueue_update = [&](cudaStream_t q) -> int {
+        BK_LAUNCH(launch_backsolve(kp, q));
+        BK_LAUNCH(launch_axpy(prec, 0, bb.V, n, kp, kp.y, 1.0, NJ_NCOL, xs, 0, 1, nax, GATE_NONE, q));
+        return enqueue_begin(q);
+    };
+    // capture [steps while a system runs, update, next residual and decisions]
+    // once; replay per cycle
     BK_CU(cudaStreamCreateWithFlags(&bb.cap, cudaStreamNonBlocking));
-    {
-        cudaGraph_t g = nullptr;
-        BK_CU(cudaStreamBeginCapture(bb.cap, cudaStreamCaptureModeThreadLocal));
-        int e1 = enqueue_cycle(bb.cap);
-        int e2 = e1 == CG_OK ? enqueue_begin(bb.cap) : e1;
-        cudaError_t ce = cudaStreamEndCapture(bb.cap, &g);
-        if (e2 != CG_OK || ce != cudaSuccess) {
-            if (g) cudaGraphDestroy(g);
-            cudaGetLastError();
-            return e2 != CG_OK ? e2 : CG_ERR_CUDA;
-        }
-        ce = cudaGraphInstantiate(&bb.gexec, g, 0);
-        cudaGraphDestroy(g);
-        if (ce != cudaSuccess) {
-            bb.gexec = nullptr;
-            cudaGetLastError();
-            return CG_ERR_CUDA;
-        }
-    }
+    BK_TRY(cycle_graph(kp, bb.cap, enqueue_steps, enqueue_update, &bb.gexec));
     BK_CU(cudaEventCreateWithFlags(&bb.ev, cudaEventDisableTiming));
     BK_TRY(enqueue_begin(s));
     std::vector<double> done_at(nb, -1.0);

@@ -467,6 +467,20 @@ int launch_cycle_begin(const KrylovPtrs &kp, int nparts, cudaStream_t s) {
     return (int)cudaGetLastError();
 }
 
+// one warp; every system's DevState lies sys_ws bytes after the previous one's
+__global__ void k_loop_test(KrylovPtrs kp, cudaGraphConditionalHandle h) {
+    int run = 0;
+    for (int i = threadIdx.x; i < kp.nsys; i += 32)
+        run |= reinterpret_cast<const DevState *>(reinterpret_cast<const char *>(kp.st) + (long long)i * kp.sys_ws)->stop == 0;
+    run = __any_sync(0xffffffffu, run);
+    if (threadIdx.x == 0) cudaGraphSetConditional(h, run ? 1u : 0u);
+}
+
+int launch_loop_test(const KrylovPtrs &kp, cudaGraphConditionalHandle h, cudaStream_t s) {
+    k_loop_test<<<1, 32, 0, s>>>(kp, h);
+    return (int)cudaGetLastError();
+}
+
 int launch_norm2(int prec, const void *v, long long n, double *npart, unsigned int *counter, double *out, int nblk,
                  cudaStream_t s) {
     if (prec == 0) k_norm2<double2><<<nblk, 256, 0, s>>>((const double2 *)v, n, npart, counter, out);
