@@ -75,7 +75,6 @@ constexpr long long OFF_BQ2 = OFF_Q2 + 2 * HID;
 constexpr long long NPARAM = OFF_BQ2 + 2;
 
 constexpr int RED_THREADS = 256;
-constexpr int WG_TILE = 32;  // cells per shared-memory tile of the weight-gradient reductions
 
 __device__ __forceinline__ bool gated(const int *g) { return g && *(volatile const int *)g; }
 
@@ -203,69 +202,112 @@ k_lift(const RT *__restrict__ r, const float *__restrict__ chi, const float *__r
 
 // -------------------------------------------------------- column-direction DFTs
 // X[line][k2][c] = sc(k2) sum_w v[line][w][c] e^{-2 pi i w k2 / W},
-// sc(0) = s0, sc(k2 > 0) = s1.  One block (512 threads = 16 k2 x 32 c) per
-// grid line; the line is staged in shared memory as FP32.
-__global__ void __launch_bounds__(512)
-k_dft_w_fwd(const __nv_bfloat16 *__restrict__ v, int W, const float2 *__restrict__ tw, float2 *__restrict__ X,
-            float s0, float s1, const int *gate) {
+// sc(0) = s0, sc(k2 > 0) = s1.  A block owns two grid lines; lane = channel, warp =
+// four column frequencies.  One 8-byte read of both lines' values and two uniform
+// 16-byte reads of the [w][16] twiddle row (all from shared memory, DW_CHUNK
+// cells at a time) feed 16 fused multiply-adds.  One frequency per thread read a
+// value, a twiddle and its index for two of them and was bound by those reads
+// (1024 lines of 64 / 256 cells: 14.7 / 45 us, now 8.8 / 26).  Per output the sum
+// runs over w in order.
+constexpr int DW_CHUNK = 64;
+__global__ void __launch_bounds__(128)
+k_dft_w_fwd(const __nv_bfloat16 *__restrict__ v, int W, long long lines, const float4 *__restrict__ twk,
+            float2 *__restrict__ X, float s0, float s1, const int *gate) {
     if (gated(gate)) return;
-    extern __shared__ float smf[];
-    float *line = smf;                              // [W][C]
-    float2 *t = reinterpret_cast<float2 *>(smf + (size_t)W * C);  // [W]
-    const long long ln = blockIdx.x;
-    const uint4 *src = reinterpret_cast<const uint4 *>(v + ln * (long long)W * C);
-    for (int q = threadIdx.x; q < W * C / 8; q += blockDim.x) {
-        const uint4 u = src[q];
-        const float2 a = unpack2(u.x), b = unpack2(u.y), c = unpack2(u.z), d = unpack2(u.w);
-        float *o = line + (size_t)q * 8;
-        o[0] = a.x, o[1] = a.y, o[2] = b.x, o[3] = b.y, o[4] = c.x, o[5] = c.y, o[6] = d.x, o[7] = d.y;
+    __shared__ float2 x[DW_CHUNK][C];  // (line 0, line 1)
+    __shared__ float4 tw[DW_CHUNK][M2 / 2];
+    const int c = threadIdx.x & 31, kg = threadIdx.x >> 5;
+    const long long ln0 = 2 * (long long)blockIdx.x, ln1 = ln0 + 1 < lines ? ln0 + 1 : ln0;
+    float2 a0[4], a1[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) a0[q] = a1[q] = make_float2(0.f, 0.f);
+    for (int w0 = 0; w0 < W; w0 += DW_CHUNK) {
+        const int nw = W - w0 < DW_CHUNK ? W - w0 : DW_CHUNK;
+        __syncthreads();
+        const uint4 *s0p = reinterpret_cast<const uint4 *>(v + (ln0 * W + w0) * C);
+        const uint4 *s1p = reinterpret_cast<const uint4 *>(v + (ln1 * W + w0) * C);
+#pragma unroll 2
+        for (int q = threadIdx.x; q < nw * C / 8; q += 128) {
+            const uint4 u = s0p[q], z = s1p[q];
+            float4 *o = reinterpret_cast<float4 *>(&x[0][0] + (size_t)q * 8);
+            float2 p = unpack2(u.x), r = unpack2(z.x);
+            o[0] = make_float4(p.x, r.x, p.y, r.y);
+            p = unpack2(u.y), r = unpack2(z.y);
+            o[1] = make_float4(p.x, r.x, p.y, r.y);
+            p = unpack2(u.z), r = unpack2(z.z);
+            o[2] = make_float4(p.x, r.x, p.y, r.y);
+            p = unpack2(u.w), r = unpack2(z.w);
+            o[3] = make_float4(p.x, r.x, p.y, r.y);
+        }
+        for (int q = threadIdx.x; q < nw * (M2 / 2); q += 128) (&tw[0][0])[q] = twk[w0 * (M2 / 2) + q];
+        __syncthreads();
+#pragma unroll 4
+        for (int w = 0; w < nw; w++) {
+            const float2 xv = x[w][c];
+            const float4 e01 = tw[w][2 * kg], e23 = tw[w][2 * kg + 1];
+            const float2 e[4] = {make_float2(e01.x, e01.y), make_float2(e01.z, e01.w), make_float2(e23.x, e23.y),
+                                 make_float2(e23.z, e23.w)};
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                a0[q].x = fmaf(xv.x, e[q].x, a0[q].x);
+                a0[q].y = fmaf(-xv.x, e[q].y, a0[q].y);
+                a1[q].x = fmaf(xv.y, e[q].x, a1[q].x);
+                a1[q].y = fmaf(-xv.y, e[q].y, a1[q].y);
+            }
+        }
     }
-    for (int m = threadIdx.x; m < W; m += blockDim.x) t[m] = tw[m];
-    __syncthreads();
-    const int k2 = threadIdx.x >> 5, c = threadIdx.x & 31;
-    float re = 0.f, im = 0.f;
-    int idx = 0;
-    for (int w = 0; w < W; w++) {
-        const float x = line[w * C + c];
-        const float2 e = t[idx];
-        re = fmaf(x, e.x, re);
-        im = fmaf(-x, e.y, im);
-        idx += k2;
-        if (idx >= W) idx -= W;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const int k2 = 4 * kg + q;
+        const float sc = k2 == 0 ? s0 : s1;
+        X[(ln0 * M2 + k2) * C + c] = make_float2(a0[q].x * sc, a0[q].y * sc);
+        if (ln1 != ln0) X[(ln1 * M2 + k2) * C + c] = make_float2(a1[q].x * sc, a1[q].y * sc);
     }
-    const float sc = k2 == 0 ? s0 : s1;
-    X[(ln * M2 + k2) * C + c] = make_float2(re * sc, im * sc);
 }
 
 // out[line][w][c] = sum_k2 sc(k2) Re(Y[line][k2][c] e^{+2 pi i w k2 / W}).
-__global__ void __launch_bounds__(256)
-k_dft_w_inv(const float2 *__restrict__ Y, int W, const float2 *__restrict__ tw, float *__restrict__ out, float s0,
-            float s1, const int *gate) {
+// Lane = channel; a thread keeps its channel's 16 scaled modes of two lines in
+// registers and walks w, reading the [w][16] twiddle row from shared memory with
+// uniform 16-byte reads: 8 of them for 64 fused multiply-adds (1024 lines of 64 /
+// 256 cells: 14.5 / 41 us with a read and its index per term, now 9.3 / 24; through
+// the read-only cache instead 23 at 256 of one line a warp).
+__global__ void __launch_bounds__(128)
+k_dft_w_inv(const float2 *__restrict__ Y, int W, long long lines, const float4 *__restrict__ twk,
+            float *__restrict__ out, float s0, float s1, const int *gate) {
     if (gated(gate)) return;
-    extern __shared__ float smf[];
-    float2 *y = reinterpret_cast<float2 *>(smf);  // [M2][C]
-    float2 *t = y + NJ;                            // [W]
-    const long long ln = blockIdx.x;
-    for (int q = threadIdx.x; q < NJ; q += blockDim.x) {
-        const float2 a = Y[ln * NJ + q];
-        const float sc = (q / C) == 0 ? s0 : s1;
-        y[q] = make_float2(a.x * sc, a.y * sc);
-    }
-    for (int m = threadIdx.x; m < W; m += blockDim.x) t[m] = tw[m];
-    __syncthreads();
+    __shared__ float4 tw[DW_CHUNK][M2 / 2];
+    const long long ln0 = 2 * (long long)blockIdx.x, ln1 = ln0 + 1 < lines ? ln0 + 1 : ln0;
     const int c = threadIdx.x & 31;
-    for (int w = threadIdx.x >> 5; w < W; w += blockDim.x >> 5) {
-        float acc = 0.f;
-        int idx = 0;
+    float2 y0[M2], y1[M2];
 #pragma unroll
-        for (int k2 = 0; k2 < M2; k2++) {
-            const float2 a = y[k2 * C + c], e = t[idx];
-            acc = fmaf(a.x, e.x, acc);
-            acc = fmaf(-a.y, e.y, acc);
-            idx += w;
-            if (idx >= W) idx -= W;
+    for (int k2 = 0; k2 < M2; k2++) {
+        const float2 a = Y[ln0 * NJ + k2 * C + c], b = Y[ln1 * NJ + k2 * C + c];
+        const float sc = k2 == 0 ? s0 : s1;
+        y0[k2] = make_float2(a.x * sc, a.y * sc);
+        y1[k2] = make_float2(b.x * sc, b.y * sc);
+    }
+    for (int w0 = 0; w0 < W; w0 += DW_CHUNK) {
+        const int nw = W - w0 < DW_CHUNK ? W - w0 : DW_CHUNK;
+        __syncthreads();
+        for (int q = threadIdx.x; q < nw * (M2 / 2); q += 128) (&tw[0][0])[q] = twk[w0 * (M2 / 2) + q];
+        __syncthreads();
+        for (int w = threadIdx.x >> 5; w < nw; w += 4) {
+            float r0 = 0.f, r1 = 0.f;
+#pragma unroll
+            for (int q = 0; q < M2 / 2; q++) {
+                const float4 e = tw[w][q];
+                r0 = fmaf(y0[2 * q].x, e.x, r0);
+                r1 = fmaf(y1[2 * q].x, e.x, r1);
+                r0 = fmaf(-y0[2 * q].y, e.y, r0);
+                r1 = fmaf(-y1[2 * q].y, e.y, r1);
+                r0 = fmaf(y0[2 * q + 1].x, e.z, r0);
+                r1 = fmaf(y1[2 * q + 1].x, e.z, r1);
+                r0 = fmaf(-y0[2 * q + 1].y, e.w, r0);
+                r1 = fmaf(-y1[2 * q + 1].y, e.w, r1);
+            }
+            out[(ln0 * W + w0 + w) * C + c] = r0;
+            if (ln1 != ln0) out[(ln1 * W + w0 + w) * C + c] = r1;
         }
-        out[(ln * W + w) * C + c] = acc;
     }
 }
 
@@ -274,6 +316,47 @@ k_dft_w_inv(const float2 *__restrict__ Y, int W, const float2 *__restrict__ tw, 
 //   P[b][hc][i][j] = sum_{h in chunk} X[b][h][j] e^{-2 pi i h k1_i / H},
 // k1_i = i (i < 16), H - 32 + i (i >= 16).  With q = 0..16 and
 // w_q = e^{+2 pi i q h / H}: k1 = q uses conj(w_q), k1 = H - q uses w_q.
+// The 17 values of q are split over blockIdx.z (Q0 <= q < Q1), and four rows are
+// loaded at a time: with all 32 sums in one thread a 16 x 64 x 64 batch filled
+// 128 blocks of 4 warps that waited for one row after another (25 us, now 14).
+template <int Q0, int Q1>
+__device__ __forceinline__ void dft_h_fwd(const float2 *__restrict__ X, int H, int h0, int h1, const float2 *tws,
+                                          float2 *__restrict__ dst) {
+    float2 lo[Q1 - Q0], hi[Q1 - Q0];  // frequencies q and H - q
+#pragma unroll
+    for (int i = 0; i < Q1 - Q0; i++) lo[i] = hi[i] = make_float2(0.f, 0.f);
+    for (int hb = h0; hb < h1; hb += 4) {
+        float2 xr[4];
+#pragma unroll
+        for (int r = 0; r < 4; r++) xr[r] = hb + r < h1 ? X[(long long)(hb + r) * NJ] : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            const int h = hb + r;
+            if (h >= h1) break;
+            const float2 x = xr[r];
+            int id = (int)((long long)Q0 * h % H);
+#pragma unroll
+            for (int q = Q0; q < Q1; q++) {
+                const float2 e = tws[id];
+                if (q < M1) {  // x * conj(e)
+                    lo[q - Q0].x += x.x * e.x + x.y * e.y;
+                    lo[q - Q0].y += x.y * e.x - x.x * e.y;
+                }
+                if (q >= 1) {  // x * e, frequency H - q (slot K1N - q)
+                    hi[q - Q0].x += x.x * e.x - x.y * e.y;
+                    hi[q - Q0].y += x.y * e.x + x.x * e.y;
+                }
+                id += h;
+                if (id >= H) id -= H;
+            }
+        }
+    }
+#pragma unroll
+    for (int q = Q0; q < Q1; q++) {
+        if (q < M1) dst[(long long)q * NJ] = lo[q - Q0];
+        if (q >= 1) dst[(long long)(K1N - q) * NJ] = hi[q - Q0];
+    }
+}
 __global__ void __launch_bounds__(128)
 k_dft_h_fwd(const float2 *__restrict__ X, int H, int HC, const float2 *__restrict__ twh, float2 *__restrict__ P,
             const int *gate) {
@@ -283,34 +366,20 @@ k_dft_h_fwd(const float2 *__restrict__ X, int H, int HC, const float2 *__restric
     __syncthreads();
     const int b = blockIdx.x / HC, hc = blockIdx.x % HC;
     const int j = blockIdx.y * 128 + threadIdx.x;
-    float2 acc[K1N];
-#pragma unroll
-    for (int i = 0; i < K1N; i++) acc[i] = make_float2(0.f, 0.f);
     const int h0 = hc * HCH, h1 = min(H, h0 + HCH);
-    for (int h = h0; h < h1; h++) {
-        const float2 x = X[((long long)b * H + h) * NJ + j];
-        int id = 0;
-#pragma unroll
-        for (int q = 0; q <= M1; q++) {
-            const float2 e = tws[id];
-            if (q < M1) {  // x * conj(e)
-                acc[q].x += x.x * e.x + x.y * e.y;
-                acc[q].y += x.y * e.x - x.x * e.y;
-            }
-            if (q >= 1) {  // x * e, frequency H - q (slot K1N - q)
-                acc[K1N - q].x += x.x * e.x - x.y * e.y;
-                acc[K1N - q].y += x.y * e.x + x.x * e.y;
-            }
-            id += h;
-            if (id >= H) id -= H;
-        }
-    }
+    const float2 *x = X + (long long)b * H * NJ + j;
     float2 *dst = P + ((long long)(b * HC + hc) * K1N) * NJ + j;
-#pragma unroll
-    for (int i = 0; i < K1N; i++) dst[(long long)i * NJ] = acc[i];
+    switch (blockIdx.z) {
+        case 0: dft_h_fwd<0, 5>(x, H, h0, h1, tws, dst); break;
+        case 1: dft_h_fwd<5, 9>(x, H, h0, h1, tws, dst); break;
+        case 2: dft_h_fwd<9, 13>(x, H, h0, h1, tws, dst); break;
+        default: dft_h_fwd<13, 17>(x, H, h0, h1, tws, dst); break;
+    }
 }
 
-// Y1[b][h][j] = sum_i Y2[b][i][j] e^{+2 pi i h k1_i / H}.
+// Y1[b][h][j] = sum_i Y2[b][i][j] e^{+2 pi i h k1_i / H}; HINV rows per block (32 rows
+// left 128 blocks for 16 x 64 x 64 cells: 13 us, now 10).
+constexpr int HINV = 8;
 __global__ void __launch_bounds__(128)
 k_dft_h_inv(const float2 *__restrict__ Y2, int H, int HC, const float2 *__restrict__ twh, float2 *__restrict__ Y1,
             const int *gate) {
@@ -323,7 +392,7 @@ k_dft_h_inv(const float2 *__restrict__ Y2, int H, int HC, const float2 *__restri
     float2 y[K1N];
 #pragma unroll
     for (int i = 0; i < K1N; i++) y[i] = Y2[((long long)b * K1N + i) * NJ + j];
-    const int h0 = hc * HCH, h1 = min(H, h0 + HCH);
+    const int h0 = hc * HINV, h1 = min(H, h0 + HINV);
     for (int h = h0; h < h1; h++) {
         float2 acc = make_float2(0.f, 0.f);
         int id = 0;
@@ -393,10 +462,10 @@ k_mix_bwd(const float2 *__restrict__ P, int B, int HC, const float *__restrict__
           const float2 *__restrict__ X2, float2 *__restrict__ dX2, float *__restrict__ grad, const int *gate) {
     if (gated(gate)) return;
     const int mode = blockIdx.x, i = mode / M2, k2 = mode % M2;
-    __shared__ float2 R[C * C];
+    __shared__ float2 R[C * (C + 1)];  // lanes read down a column: odd pitch
     __shared__ float2 dys[8][C], xs[8][C];
     const float2 *Rg = reinterpret_cast<const float2 *>(prm + off_r(layer)) + (long long)mode * C * C;
-    for (int q = threadIdx.x; q < C * C; q += blockDim.x) R[q] = Rg[q];
+    for (int q = threadIdx.x; q < C * C; q += blockDim.x) R[q / C * (C + 1) + q % C] = Rg[q];
     const int lane = threadIdx.x & 31, bl = threadIdx.x >> 5;
     float2 dr[4];
 #pragma unroll
@@ -421,7 +490,7 @@ k_mix_bwd(const float2 *__restrict__ P, int B, int HC, const float *__restrict__
             float2 acc = make_float2(0.f, 0.f);
 #pragma unroll 8
             for (int o = 0; o < C; o++) {
-                const float2 d = dys[bl][o], r = R[lane * C + o];
+                const float2 d = dys[bl][o], r = R[lane * (C + 1) + o];
                 acc.x += d.x * r.x + d.y * r.y;
                 acc.y += d.y * r.x - d.x * r.y;
             }
@@ -742,116 +811,264 @@ __global__ void k_dout_from_dm(float *__restrict__ o, const cg_c64 *__restrict__
     }
 }
 
-// Projection backward on the CUDA cores: thread j = hidden unit over a chunk
-// of cells: dzq = (Q2^T do) GELU'(zq); partials of dQ2 = sum do GELU(zq)^T and
-// dbq2 = sum do.  Partial layout per block: [Q2 (2 x HID), bq2 (2)].
-__global__ void __launch_bounds__(HID)
+// Projection backward on the CUDA cores: thread = hidden unit j, PB_GROUPS groups
+// of HID threads share a block's cells: dzq = (Q2^T do) GELU'(zq); partials of
+// dQ2 = sum do GELU(zq)^T and dbq2 = sum do.  Partial layout per block:
+// [Q2 (2 x HID), bq2 (2)].  Bound by the error function and the exponential of
+// each value; one group of 4 warps per block of 256 cells left the SMs with 7
+// warps (16 x 64 x 64 cells: 98 us, now 28).
+constexpr int PB_GROUPS = 4;
+__global__ void __launch_bounds__(HID *PB_GROUPS)
 k_proj_bwd(const __nv_bfloat16 *__restrict__ zq, const float *__restrict__ dout, const float *__restrict__ prm,
            long long cells, __nv_bfloat16 *__restrict__ dzq, float *__restrict__ part) {
-    const int j = threadIdx.x;
+    __shared__ float sum[PB_GROUPS][2 * HID + 2];
+    const int j = threadIdx.x % HID, g = threadIdx.x / HID;
     const float w0 = prm[OFF_Q2 + j], w1 = prm[OFF_Q2 + HID + j];
     const long long per = (cells + gridDim.x - 1) / gridDim.x;
     const long long e0 = (long long)blockIdx.x * per, e1 = min(cells, e0 + per);
     float a0 = 0.f, a1 = 0.f, b0 = 0.f, b1 = 0.f;
-    for (long long e = e0; e < e1; e++) {
+#pragma unroll 4
+    for (long long e = e0 + g; e < e1; e += PB_GROUPS) {
         const float z = __bfloat162float(zq[e * HID + j]);
         const float d0 = dout[2 * e], d1 = dout[2 * e + 1];
-        const float g = gelu(z);
-        a0 = fmaf(d0, g, a0);
-        a1 = fmaf(d1, g, a1);
+        const float gz = gelu(z);
+        a0 = fmaf(d0, gz, a0);
+        a1 = fmaf(d1, gz, a1);
         if (j == 0) b0 += d0, b1 += d1;
         dzq[e * HID + j] = __float2bfloat16_rn((w0 * d0 + w1 * d1) * gelu_d(z));
     }
+    sum[g][j] = a0;
+    sum[g][HID + j] = a1;
+    if (j == 0) sum[g][2 * HID] = b0, sum[g][2 * HID + 1] = b1;
+    __syncthreads();
     float *p = part + (long long)blockIdx.x * (2 * HID + 2);
-    p[j] = a0;
-    p[HID + j] = a1;
-    if (j == 0) p[2 * HID] = b0, p[2 * HID + 1] = b1;
+    if (threadIdx.x < 2 * HID + 2) {
+        float t = 0.f;
+#pragma unroll
+        for (int q = 0; q < PB_GROUPS; q++) t += sum[q][threadIdx.x];
+        p[threadIdx.x] = t;
+    }
 }
 
 // Weight gradient of a channel mixing: dWt[o][i] = sum_cells dY[o] X[i],
-// db[o] = sum_cells dY[o]; per-block partials [NO*NI + NO].
-template <int NO, int NI>
-__global__ void __launch_bounds__(RED_THREADS)
+// db[o] = sum_cells dY[o]; per-block partials [NO*NI + NO].  A contraction over
+// the cells of two BF16 arrays, so it runs on the tensor cores (mma.sync m16n8k16,
+// FP32 accumulators; the operands are cell-major, which ldmatrix.trans turns into
+// fragments).  mma.sync and not tcgen05: the outputs are one 32- or 128-row tile
+// that a warp's registers hold, and the kernel is bound by reading the cells
+// once.  Tiles of 64 cells, double-buffered with cp.async.  NO = 128: warp w owns
+// rows 32 w ..; NO = 32: warp w takes every fourth group of 16 cells and the block
+// adds the warps' tiles in order.  db is one more column tile against ones.
+// 16 x 64 x 64 cells: 74 -> 8 us (NO = 128) and 45 -> 6 us (NO = 32) against FP32
+// fused multiply-adds from shared memory.
+constexpr int WG_CELLS = 64, WG_THREADS = 128;
+__device__ __forceinline__ uint32_t wg_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void wg_copy16(void *dst, const void *src, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(wg_smem(dst)), "l"(src), "r"(ok ? 16 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void wg_ldsm_t(uint32_t (&r)[4], const __nv_bfloat16 *row) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(wg_smem(row)));
+}
+__device__ __forceinline__ void wg_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+                 "{%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+template <int NO>
+__global__ void __launch_bounds__(WG_THREADS)
 k_wgrad(const __nv_bfloat16 *__restrict__ dY, const __nv_bfloat16 *__restrict__ X, long long cells,
         float *__restrict__ part) {
-    constexpr int PER = NO * NI / RED_THREADS;  // outputs per thread (4 or 16), same o, consecutive i
-    static_assert(NO * NI % RED_THREADS == 0 && NI % PER == 0, "shape");
-    __shared__ float sd[WG_TILE][NO + 1];
-    __shared__ float sx[WG_TILE][NI + 4];
-    const int t = threadIdx.x;
-    const int o = (t * PER) / NI, i0 = (t * PER) % NI;
-    float acc[PER];
-#pragma unroll
-    for (int q = 0; q < PER; q++) acc[q] = 0.f;
-    float bacc = 0.f;
-    const long long ntile = (cells + WG_TILE - 1) / WG_TILE;
-    for (long long tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
-        const long long c0 = tile * WG_TILE;
+    constexpr int NI = C, LD = NO + 8, LX = NI + 8;  // row pitches: an odd number of 16-byte units
+    constexpr int SD = WG_CELLS * LD, SX = WG_CELLS * LX;
+    static_assert(NO == 32 || NO == 128, "four warps");
+    __shared__ __align__(16) __nv_bfloat16 sm[2 * (SD + SX)];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int m0 = NO == 128 ? 32 * warp : 0;
+    float acc[2][5][4] = {};  // 16-row tiles x (four 8-column tiles, the sum column)
+    const long long ntile = (cells + WG_CELLS - 1) / WG_CELLS;
+    auto issue = [&](long long tile, int buf) {
+        __nv_bfloat16 *d = sm + buf * (SD + SX), *x = d + SD;
+        const long long c0 = tile * WG_CELLS;
+        for (int q = threadIdx.x; q < WG_CELLS * NO / 8; q += WG_THREADS) {
+            const int rr = q / (NO / 8), cc = q % (NO / 8) * 8;
+            const bool ok = c0 + rr < cells;
+            wg_copy16(d + rr * LD + cc, dY + (ok ? c0 + rr : 0) * NO + cc, ok);
+        }
+        for (int q = threadIdx.x; q < WG_CELLS * NI / 8; q += WG_THREADS) {
+            const int rr = q / (NI / 8), cc = q % (NI / 8) * 8;
+            const bool ok = c0 + rr < cells;
+            wg_copy16(x + rr * LX + cc, X + (ok ? c0 + rr : 0) * NI + cc, ok);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    long long tile = blockIdx.x;
+    if (tile < ntile) issue(tile, 0);
+    for (int it = 0; tile < ntile; it++, tile += gridDim.x) {
+        if (tile + gridDim.x < ntile) {
+            issue(tile + gridDim.x, (it + 1) & 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
         __syncthreads();
-        for (int q = t; q < WG_TILE * NO; q += RED_THREADS) {
-            const int rr = q / NO, cc = q % NO;
-            sd[rr][cc] = c0 + rr < cells ? __bfloat162float(dY[(c0 + rr) * NO + cc]) : 0.f;
-        }
-        for (int q = t; q < WG_TILE * NI; q += RED_THREADS) {
-            const int rr = q / NI, cc = q % NI;
-            sx[rr][cc] = c0 + rr < cells ? __bfloat162float(X[(c0 + rr) * NI + cc]) : 0.f;
-        }
-        __syncthreads();
-#pragma unroll 4
-        for (int rr = 0; rr < WG_TILE; rr++) {
-            const float d = sd[rr][o];
+        const __nv_bfloat16 *d = sm + (it & 1) * (SD + SX), *x = d + SD;
 #pragma unroll
-            for (int q = 0; q < PER; q++) acc[q] = fmaf(d, sx[rr][i0 + q], acc[q]);
+        for (int ks = 0; ks < WG_CELLS / 16; ks++) {
+            if (NO == 32 && ks != warp) continue;
+            const int k0 = 16 * ks;
+            // A: 8 x 8 blocks (rows, cells) = (0, 0), (8, 0), (0, 8), (8, 8); B: (cells, columns) = (0, 0), (8, 0), (0, 8), (8, 8)
+            uint32_t a[2][4], b[2][4];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                wg_ldsm_t(a[h], d + (k0 + (lane & 7) + (lane >> 4) * 8) * LD + m0 + 16 * h + ((lane >> 3) & 1) * 8);
+                wg_ldsm_t(b[h], x + (k0 + (lane & 15)) * LX + 16 * h + (lane >> 4) * 8);
+            }
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+#pragma unroll
+                for (int n = 0; n < 4; n++) wg_mma(acc[h][n], a[h], b[n >> 1][2 * (n & 1)], b[n >> 1][2 * (n & 1) + 1]);
+                wg_mma(acc[h][4], a[h], 0x3f803f80u, 0x3f803f80u);
+            }
         }
-        if (t < NO)
-            for (int rr = 0; rr < WG_TILE; rr++) bacc += sd[rr][t];
+        __syncthreads();  // the next issue refills this buffer
     }
     float *p = part + (long long)blockIdx.x * (NO * NI + NO);
+    const int r0 = lane >> 2, cq = 2 * (lane & 3);  // accumulator rows r0, r0 + 8, columns cq, cq + 1
+    if constexpr (NO == 128) {
 #pragma unroll
-    for (int q = 0; q < PER; q++) p[o * NI + i0 + q] = acc[q];
-    if (t < NO) p[NO * NI + t] = bacc;
+        for (int h = 0; h < 2; h++) {
+            const int o = m0 + 16 * h + r0;
+#pragma unroll
+            for (int n = 0; n < 4; n++) {
+                p[o * NI + 8 * n + cq] = acc[h][n][0];
+                p[o * NI + 8 * n + cq + 1] = acc[h][n][1];
+                p[(o + 8) * NI + 8 * n + cq] = acc[h][n][2];
+                p[(o + 8) * NI + 8 * n + cq + 1] = acc[h][n][3];
+            }
+            if (cq == 0) {
+                p[NO * NI + o] = acc[h][4][0];
+                p[NO * NI + o + 8] = acc[h][4][2];
+            }
+        }
+    } else {
+        constexpr int LS = NI + 1;
+        static_assert(4 * NO * LS * sizeof(float) <= sizeof(sm), "the warps' tiles fit the staging buffer");
+        float *st = reinterpret_cast<float *>(sm) + warp * NO * LS;
+        __syncthreads();
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int o = 16 * h + r0;
+#pragma unroll
+            for (int n = 0; n < 4; n++) {
+                st[o * LS + 8 * n + cq] = acc[h][n][0];
+                st[o * LS + 8 * n + cq + 1] = acc[h][n][1];
+                st[(o + 8) * LS + 8 * n + cq] = acc[h][n][2];
+                st[(o + 8) * LS + 8 * n + cq + 1] = acc[h][n][3];
+            }
+            if (cq == 0) {
+                st[o * LS + NI] = acc[h][4][0];
+                st[(o + 8) * LS + NI] = acc[h][4][2];
+            }
+        }
+        __syncthreads();
+        const float *all = reinterpret_cast<const float *>(sm);
+        for (int q = threadIdx.x; q < NO * LS; q += WG_THREADS) {
+            const float t = ((all[q] + all[NO * LS + q]) + all[2 * NO * LS + q]) + all[3 * NO * LS + q];
+            const int o = q / LS, i = q % LS;
+            p[i < NI ? o * NI + i : NO * NI + o] = t;
+        }
+    }
 }
 
-// Lift backward: dP[c][j] = sum dv0[c] f_j, dpb[c] = sum dv0[c]; thread (c, j).
+// Lift backward: dP[c][j] = sum dv0[c] f_j, dpb[c] = sum dv0[c].  Lane = channel;
+// a warp takes 32 cells at a time, whose features its lanes load side by side and
+// hand round by shuffles, so every load is coalesced and eight rows of dv0 are in
+// flight (a thread per (c, j) walking its block's cells took 163 us on 16 x 64 x 64
+// cells, bound by one load's latency per cell).
 template <typename RT>
-__global__ void __launch_bounds__(C * NIN)
+__global__ void __launch_bounds__(RED_THREADS)
 k_lift_bwd(const float *__restrict__ dv0, const RT *__restrict__ r, const float *__restrict__ chi,
            const float *__restrict__ k0h, const float *__restrict__ inv_s, long long hw, long long cells,
            float *__restrict__ part) {
-    const int c = threadIdx.x >> 2, jf = threadIdx.x & 3;
-    const long long per = (cells + gridDim.x - 1) / gridDim.x;
-    const long long e0 = (long long)blockIdx.x * per, e1 = min(cells, e0 + per);
-    float a = 0.f, bsum = 0.f;
-    for (long long e = e0; e < e1; e++) {
-        const int b = (int)(e / hw);
-        const float d = dv0[e * C + c];
-        float f;
-        if (jf == 0) f = chi[e] * CHI_SCALE;
-        else if (jf == 1) f = k0h[b];
-        else if (jf == 2) f = re_of(r[e]) * inv_s[b];
-        else f = im_of(r[e]) * inv_s[b];
-        a = fmaf(d, f, a);
-        if (jf == 0) bsum += d;
+    constexpr int NW = RED_THREADS / 32;
+    static_assert(NIN == 4, "features");
+    __shared__ float acc[NW][NIN + 1][C];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float a[NIN + 1] = {};
+    for (long long g = ((long long)blockIdx.x * NW + warp) * 32; g < cells; g += (long long)gridDim.x * NW * 32) {
+        const long long e = g + lane;
+        const int n = (int)(cells - g < 32 ? cells - g : 32);
+        float f0 = 0.f, f1 = 0.f, f2 = 0.f, f3 = 0.f;
+        if (lane < n) {
+            const int b = (int)(e / hw);
+            const RT v = r[e];
+            f0 = chi[e] * CHI_SCALE;
+            f1 = k0h[b];
+            f2 = re_of(v) * inv_s[b];
+            f3 = im_of(v) * inv_s[b];
+        }
+#pragma unroll
+        for (int q0 = 0; q0 < 32; q0 += 8) {
+            float d[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) d[q] = q0 + q < n ? dv0[(g + q0 + q) * C + lane] : 0.f;
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                a[0] = fmaf(d[q], __shfl_sync(0xffffffffu, f0, q0 + q), a[0]);
+                a[1] = fmaf(d[q], __shfl_sync(0xffffffffu, f1, q0 + q), a[1]);
+                a[2] = fmaf(d[q], __shfl_sync(0xffffffffu, f2, q0 + q), a[2]);
+                a[3] = fmaf(d[q], __shfl_sync(0xffffffffu, f3, q0 + q), a[3]);
+                a[4] += d[q];
+            }
+        }
     }
+#pragma unroll
+    for (int j = 0; j <= NIN; j++) acc[warp][j][lane] = a[j];
+    __syncthreads();
     float *p = part + (long long)blockIdx.x * (C * NIN + C);
-    p[c * NIN + jf] = a;
-    if (jf == 0) p[C * NIN + c] = bsum;
+    if (threadIdx.x < C * (NIN + 1)) {
+        const int j = threadIdx.x / C, c = threadIdx.x % C;
+        float t = 0.f;
+        for (int w = 0; w < NW; w++) t += acc[w][j][c];
+        p[j < NIN ? c * NIN + j : C * NIN + c] = t;
+    }
 }
 
-// dst[i] = sum_b part[b][i] (fixed order).
-__global__ void k_reduce(const float *__restrict__ part, int nblk, int cnt, float *__restrict__ dst) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
-        double s = 0.0;
-        for (int b = 0; b < nblk; b++) s += part[(long long)b * cnt + i];
-        dst[i] = (float)s;
+// dst[i] = sum_b part[b][i] (fixed order).  A block owns 32 outputs; its 32 warps
+// share the partial rows, so that a few hundred rows are a dozen loads deep: one
+// thread per output walked them in 35 us, whatever their size (now 3 to 5 us).
+constexpr int REDUCE_ROWS = 32;
+__global__ void __launch_bounds__(32 * REDUCE_ROWS) k_reduce(const float *__restrict__ part, int nblk, int cnt,
+                                                             float *__restrict__ dst) {
+    __shared__ double sum[REDUCE_ROWS][33];
+    const int x = threadIdx.x & 31, y = threadIdx.x >> 5, i = blockIdx.x * 32 + x;
+    double s = 0.0;
+    if (i < cnt) {
+#pragma unroll 8
+        for (int b = y; b < nblk; b += REDUCE_ROWS) s += part[(long long)b * cnt + i];
+    }
+    sum[y][x] = s;
+    __syncthreads();
+    if (y == 0 && i < cnt) {
+        double t = 0.0;
+#pragma unroll
+        for (int q = 0; q < REDUCE_ROWS; q++) t += sum[q][x];
+        dst[i] = (float)t;
     }
 }
+void reduce(const float *part, int nblk, int cnt, float *dst, cudaStream_t s) {
+    k_reduce<<<(cnt + 31) / 32, 32 * REDUCE_ROWS, 0, s>>>(part, nblk, cnt, dst);
+}
+// one warp; fixed order
 __global__ void k_reduce_d(const double *__restrict__ part, int nblk, double *__restrict__ dst) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double s = 0.0;
-        for (int b = 0; b < nblk; b++) s += part[b];
-        *dst = s;
-    }
+    double s = 0.0;
+    for (int b = threadIdx.x; b < nblk; b += 32) s += part[b];
+    s = warp_sum(s);
+    if (threadIdx.x == 0) *dst = s;
 }
 
 // ---------------------------------------------------------------- optimiser
@@ -993,7 +1210,8 @@ struct cg_fno {
     CUtensorMap mapVT, mapTwHi, mapTwLo, mapTwInv;
     // twiddles of the current grid
     int tw_H = 0, tw_W = 0;
-    float2 *twh = nullptr, *tww = nullptr;
+    float2 *twh = nullptr;
+    float4 *twk = nullptr;  // [w][16] e^{2 pi i w k / W}, two per entry
     float apply_k0h = -1.f;  // k0 h held in k0h[0] for single-vector applications
     bool local_last = true;  // false: the last Fourier layer has no pointwise path (W_3 unused, held at 0)
     int fwd_B = 0, fwd_H = 0, fwd_W = 0;  // batch kept by cugmres_fno_forward_train
@@ -1131,17 +1349,20 @@ int ensure_maps(cg_fno *f, long long cells) {
 int ensure_twiddles(cg_fno *f, int H, int W) {
     if (f->tw_H == H && f->tw_W == W) return CG_OK;
     if (f->twh) cudaFree(f->twh);
-    if (f->tww) cudaFree(f->tww);
-    f->twh = f->tww = nullptr;
+    if (f->twk) cudaFree(f->twk);
+    f->twh = nullptr;
+    f->twk = nullptr;
     f->tw_H = f->tw_W = 0;
-    std::vector<float2> th(H), tw(W);
+    std::vector<float2> th(H), tw(W), twk((size_t)W * M2);
     const double pi = 3.14159265358979323846;
     for (int m = 0; m < H; m++) th[m] = make_float2((float)cos(2 * pi * m / H), (float)sin(2 * pi * m / H));
     for (int m = 0; m < W; m++) tw[m] = make_float2((float)cos(2 * pi * m / W), (float)sin(2 * pi * m / W));
+    for (int w = 0; w < W; w++)
+        for (int k = 0; k < M2; k++) twk[(size_t)w * M2 + k] = tw[(size_t)w * k % W];
     FN_CU(cudaMalloc(&f->twh, sizeof(float2) * H));
-    FN_CU(cudaMalloc(&f->tww, sizeof(float2) * W));
+    FN_CU(cudaMalloc(&f->twk, sizeof(float2) * twk.size()));
     FN_CU(cudaMemcpyAsync(f->twh, th.data(), sizeof(float2) * H, cudaMemcpyHostToDevice, f->stream));
-    FN_CU(cudaMemcpyAsync(f->tww, tw.data(), sizeof(float2) * W, cudaMemcpyHostToDevice, f->stream));
+    FN_CU(cudaMemcpyAsync(f->twk, twk.data(), sizeof(float2) * twk.size(), cudaMemcpyHostToDevice, f->stream));
     FN_CU(cudaStreamSynchronize(f->stream));  // applications inside a solve read them on the solver's stream
     f->tw_H = H;
     f->tw_W = W;
@@ -1184,13 +1405,8 @@ int prepare_grid(cg_fno *f, int B, int H, int W) {
     return CG_OK;
 }
 
-size_t dft_w_fwd_smem(int W) { return (size_t)W * C * 4 + (size_t)W * 8; }
-size_t dft_w_inv_smem(int W) { return (size_t)NJ * 8 + (size_t)W * 8; }
-
-int set_smem_attrs(int W, int H) {
-    if (cudaFuncSetAttribute(k_dft_w_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dft_w_fwd_smem(W)) ||
-        cudaFuncSetAttribute(k_dft_w_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dft_w_inv_smem(W)) ||
-        cudaFuncSetAttribute(k_dft_h_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, H * 8) ||
+int set_smem_attrs(int H) {
+    if (cudaFuncSetAttribute(k_dft_h_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, H * 8) ||
         cudaFuncSetAttribute(k_dft_h_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, H * 8))
         return -1;
     return 0;
@@ -1201,7 +1417,7 @@ int set_smem_attrs(int W, int H) {
 int spectral_fwd(cg_fno *f, const __nv_bfloat16 *in, int B, int H, int W, int layer, float2 *X2save, const int *gate,
                  cudaStream_t s, bool tc) {
     const long long lines = (long long)B * H;
-    const int HC = (H + HCH - 1) / HCH;
+    const int HC = (H + HCH - 1) / HCH, HCI = (H + HINV - 1) / HINV;
     if (tc) {
         EpiDftW e;
         e.X = reinterpret_cast<float *>(f->X1);
@@ -1211,11 +1427,12 @@ int spectral_fwd(cg_fno *f, const __nv_bfloat16 *in, int B, int H, int W, int la
         e.add = 1;
         FN_K(gemm<32, 1, 6>(f->sms, f->mapVT, f->mapTwLo, lines * W, e, f->err, gate, s));
     } else {
-        k_dft_w_fwd<<<(unsigned)lines, 512, dft_w_fwd_smem(W), s>>>(in, W, f->tww, f->X1, 1.f, 1.f, gate);
+        k_dft_w_fwd<<<(unsigned)((lines + 1) / 2), 128, 0, s>>>(in, W, lines, f->twk, f->X1, 1.f, 1.f,
+                                                                                   gate);
     }
-    k_dft_h_fwd<<<dim3(B * HC, NJ / 128), 128, H * 8, s>>>(f->X1, H, HC, f->twh, f->Hp, gate);
+    k_dft_h_fwd<<<dim3(B * HC, NJ / 128, 4), 128, H * 8, s>>>(f->X1, H, HC, f->twh, f->Hp, gate);
     k_mix_fwd<<<K1N * M2, 256, 0, s>>>(f->Hp, B, HC, f->p, layer, X2save, f->Y2, gate);
-    k_dft_h_inv<<<dim3(B * HC, NJ / 128), 128, H * 8, s>>>(f->Y2, H, HC, f->twh, f->X1, gate);
+    k_dft_h_inv<<<dim3(B * HCI, NJ / 128), 128, H * 8, s>>>(f->Y2, H, HCI, f->twh, f->X1, gate);
     const float inv = 1.f / ((float)H * (float)W);
     if (tc) {
         // Z reuses the channel-major buffer (its column DFT has run) and its map
@@ -1226,7 +1443,7 @@ int spectral_fwd(cg_fno *f, const __nv_bfloat16 *in, int B, int H, int W, int la
         e.out = f->spec;
         FN_K(gemm<32, 1, 6>(f->sms, f->mapVT, f->mapTwInv, lines * W, e, f->err, gate, s));
     } else {
-        k_dft_w_inv<<<(unsigned)lines, 256, dft_w_inv_smem(W), s>>>(f->X1, W, f->tww, f->spec, inv, 2.f * inv, gate);
+        k_dft_w_inv<<<(unsigned)((lines + 1) / 2), 128, 0, s>>>(f->X1, W, lines, f->twk, f->spec, inv, 2.f * inv, gate);
     }
     return (int)cudaGetLastError();
 }
@@ -1237,8 +1454,8 @@ template <typename RT>
 int forward(cg_fno *f, cudaStream_t s, int B, int H, int W, const RT *r, const float *chi, RT *zout, bool train,
             const cg_c64 *x, const int *gate) {
     const long long hw = (long long)H * W, cells = B * hw;
-    if (set_smem_attrs(W, H)) return CG_ERR_CUDA;
-    const int nbx = (int)std::max<long long>(1, std::min<long long>(NBX_MAX, (hw + 4095) / 4096));
+    if (set_smem_attrs(H)) return CG_ERR_CUDA;
+    const int nbx = (int)std::max<long long>(1, std::min<long long>(NBX_MAX, (hw + 1023) / 1024));
     k_norm_part<RT><<<dim3(nbx, B), RED_THREADS, 0, s>>>(r, train ? x : nullptr, hw, nbx, f->npart, gate);
     k_norm_fin<<<(B + 63) / 64, 64, 0, s>>>(f->npart, nbx, B, hw, f->s, f->inv_s, train ? f->wts : nullptr, gate);
     const int lb = (int)std::min<long long>((cells + 255) / 256, 8LL * f->sms);
@@ -1283,7 +1500,7 @@ int forward(cg_fno *f, cudaStream_t s, int B, int H, int W, const RT *r, const f
 int backward(cg_fno *f, cudaStream_t s, int B, int H, int W, const cg_c64 *r, const cg_c64 *x, const float *chi,
              const cg_c64 *dm) {
     const long long hw = (long long)H * W, cells = B * hw, lines = (long long)B * H;
-    const int HC = (H + HCH - 1) / HCH;
+    const int HC = (H + HCH - 1) / HCH, HCI = (H + HINV - 1) / HINV;
     const int nred = reduction_blocks(f, cells);
     if (x) {
         double *lpart = reinterpret_cast<double *>(f->part);
@@ -1294,10 +1511,13 @@ int backward(cg_fno *f, cudaStream_t s, int B, int H, int W, const cg_c64 *r, co
     }
     FN_K(cudaGetLastError());
     // projection
-    k_proj_bwd<<<nred, HID, 0, s>>>(f->zq, f->out2, f->p, cells, f->dzq, f->part);
-    k_reduce<<<2, 256, 0, s>>>(f->part, nred, 2 * HID + 2, f->g + OFF_Q2);
-    k_wgrad<HID, C><<<nred, RED_THREADS, 0, s>>>(f->dzq, f->act[LAYERS], cells, f->part);
-    k_reduce<<<(HID * C + HID + 255) / 256, 256, 0, s>>>(f->part, nred, HID * C + HID, f->g + OFF_Q1);
+    // twice nred blocks fill the SMs (their rows of 2 HID + 2 sums fit the nred rows of HID C + HID in f->part)
+    static_assert(2 * (2 * HID + 2) <= HID * C + HID, "partial sums of k_proj_bwd");
+    const int nproj = (int)std::min<long long>(2LL * nred, (cells + 31) / 32);
+    k_proj_bwd<<<nproj, HID * PB_GROUPS, 0, s>>>(f->zq, f->out2, f->p, cells, f->dzq, f->part);
+    reduce(f->part, nproj, 2 * HID + 2, f->g + OFF_Q2, s);
+    k_wgrad<HID><<<nred, WG_THREADS, 0, s>>>(f->dzq, f->act[LAYERS], cells, f->part);
+    reduce(f->part, nred, HID * C + HID, f->g + OFF_Q1, s);
     FN_K(cudaGetLastError());
     EpiBwd eb;
     eb.dspec = nullptr;
@@ -1309,17 +1529,17 @@ int backward(cg_fno *f, cudaStream_t s, int B, int H, int W, const cg_c64 *r, co
     int cur = 0;
     const float inv = 1.f / ((float)H * (float)W);
     for (int l = LAYERS - 1; l >= 0; l--) {
-        k_wgrad<C, C><<<nred, RED_THREADS, 0, s>>>(f->dz[cur], f->act[l], cells, f->part);
-        k_reduce<<<(C * C + C + 255) / 256, 256, 0, s>>>(f->part, nred, C * C + C, f->g + off_w(l));
+        k_wgrad<C><<<nred, WG_THREADS, 0, s>>>(f->dz[cur], f->act[l], cells, f->part);
+        reduce(f->part, nred, C * C + C, f->g + off_w(l), s);
         const bool spec_only = l == LAYERS - 1 && !f->local_last;
         if (spec_only) FN_CU(cudaMemsetAsync(f->g + off_w(l), 0, sizeof(float) * C * C, s));
         // spectral adjoint: dY1 = adjoint of the inverse column DFT, then rows, modes, rows, columns
-        k_dft_w_fwd<<<(unsigned)lines, 512, dft_w_fwd_smem(W), s>>>(f->dz[cur], W, f->tww, f->X1, inv, 2.f * inv,
-                                                                      nullptr);
-        k_dft_h_fwd<<<dim3(B * HC, NJ / 128), 128, H * 8, s>>>(f->X1, H, HC, f->twh, f->Hp, nullptr);
+        k_dft_w_fwd<<<(unsigned)((lines + 1) / 2), 128, 0, s>>>(f->dz[cur], W, lines, f->twk, f->X1, inv,
+                                                                                   2.f * inv, nullptr);
+        k_dft_h_fwd<<<dim3(B * HC, NJ / 128, 4), 128, H * 8, s>>>(f->X1, H, HC, f->twh, f->Hp, nullptr);
         k_mix_bwd<<<K1N * M2, 256, 0, s>>>(f->Hp, B, HC, f->p, l, f->X2s[l], f->Y2, f->g, nullptr);
-        k_dft_h_inv<<<dim3(B * HC, NJ / 128), 128, H * 8, s>>>(f->Y2, H, HC, f->twh, f->X1, nullptr);
-        k_dft_w_inv<<<(unsigned)lines, 256, dft_w_inv_smem(W), s>>>(f->X1, W, f->tww, f->spec, 1.f, 1.f, nullptr);
+        k_dft_h_inv<<<dim3(B * HCI, NJ / 128), 128, H * 8, s>>>(f->Y2, H, HCI, f->twh, f->X1, nullptr);
+        k_dft_w_inv<<<(unsigned)((lines + 1) / 2), 128, 0, s>>>(f->X1, W, lines, f->twk, f->spec, 1.f, 1.f, nullptr);
         FN_K(cudaGetLastError());
         if (spec_only) {  // dv = dspec only; l - 1 >= 0 has GELU
             k_spec_bwd<<<nred, 256, 0, s>>>(f->spec, f->zpre[l - 1], f->dz[cur ^ 1], cells);
@@ -1343,9 +1563,9 @@ int backward(cg_fno *f, cudaStream_t s, int B, int H, int W, const cg_c64 *r, co
         FN_K(gemm<32, 1, 6>(f->sms, f->mapDZ[cur], f->mapWT[l], cells, e, f->err, nullptr, s));
         cur ^= 1;
     }
-    k_lift_bwd<float2><<<nred, C * NIN, 0, s>>>(f->spec, reinterpret_cast<const float2 *>(r), chi, f->k0h, f->inv_s,
+    k_lift_bwd<float2><<<nred, RED_THREADS, 0, s>>>(f->spec, reinterpret_cast<const float2 *>(r), chi, f->k0h, f->inv_s,
                                                 hw, cells, f->part);
-    k_reduce<<<1, 256, 0, s>>>(f->part, nred, C * NIN + C, f->g + OFF_P);
+    reduce(f->part, nred, C * NIN + C, f->g + OFF_P, s);
     FN_K(cudaGetLastError());
     return CG_OK;
 }
@@ -1483,7 +1703,7 @@ extern "C" void cugmres_fno_destroy(cg_fno *f) {
     cudaFree(f->err);
     cudaFree(f->ws);
     cudaFree(f->twh);
-    cudaFree(f->tww);
+    cudaFree(f->twk);
     if (f->stream) cudaStreamDestroy(f->stream);
     cudaGetLastError();
     delete f;

@@ -286,3 +286,28 @@ def test_fno_set_params_is_complete_on_return(cuda_device):
         twice = net.loss_grad(chi, k0h, r, x)
         net.close()
         assert once[0] == twice[0] and np.array_equal(once[1], twice[1])
+
+
+@pytest.mark.parametrize("shape", [(1, 33, 35), (3, 45, 67), (2, 70, 129), (1, 32, 33), (5, 37, 256)])
+def test_fno_ragged_grids_match_oracle(net, shape):
+    """Odd line counts, widths around the column transforms' 64-cell chunks, rows that
+    fill no whole chunk and cell counts that fill no whole tile: forward pass and
+    every gradient block against the oracle, within the bounds of BF16 storage."""
+    p = _params(4)
+    net.set_params(p)
+    chi, k0h, r, x = _inputs(*shape, 13)
+    z = net.forward(chi, k0h, r)
+    ref = FO.forward(p, chi, k0h, r, bf16=True)
+    corr_ref = ref["z"].numpy() - r
+    assert np.linalg.norm(z - ref["z"].numpy()) < 2e-2 * np.linalg.norm(corr_ref)
+    loss, g = net.loss_grad(chi, k0h, r, x)
+    loss_ref, g_ref = FO.loss_grad(p, chi, k0h, r, x, bf16=True)
+    assert abs(loss - loss_ref) <= 5e-3 * abs(loss_ref)
+    cuts = [FO.OFF_P, FO.OFF_PB, FO.OFF_L0]
+    for l in range(FO.LAYERS):
+        o = FO.off_r(l)
+        cuts += [o + FO.RSZ, o + FO.RSZ + FO.C * FO.C, o + FO.LSZ]
+    cuts += [FO.OFF_BQ1, FO.OFF_Q2, FO.OFF_BQ2, FO.NPARAM]
+    for a, b in zip(cuts[:-1], cuts[1:]):
+        e = np.linalg.norm(g[a:b] - g_ref[a:b]) / np.linalg.norm(g_ref[a:b])
+        assert e < 5e-2, (a, b, e)
