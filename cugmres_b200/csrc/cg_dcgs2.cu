@@ -243,8 +243,10 @@ __global__ void __launch_bounds__(D2_THREADS, 2) k_dots2t(const CV *__restrict__
 // w of the tile in registers.  Every coefficient j has one owning warp, so the
 // block accumulates it in a single shared-memory slot (chunks of cs vectors)
 // without atomics; block partials and the last-block sum as in k_dots2t.
-template <typename CV, int U>
-__global__ void __launch_bounds__(D2_THREADS) k_dots2s(const CV *__restrict__ V, long long n, KrylovPtrs kp) {
+// MINB blocks per SM: 2 where the tiles outnumber the SMs (148 registers had kept
+// one 8-warp block, 32 KB of loads, on an SM: 512^2 FP64 at 3.4 TB/s).
+template <typename CV, int U, int MINB = 1>
+__global__ void __launch_bounds__(D2_THREADS, MINB) k_dots2s(const CV *__restrict__ V, long long n, KrylovPtrs kp) {
     kp = kp_sys(kp);  // this block's system of a bucket
     V = sys_vec(V, kp);
     typedef typename real_of<CV>::type R;
@@ -760,8 +762,9 @@ __global__ void __launch_bounds__(AX2_THREADS, 2) k_axpy2t(CV *__restrict__ V, l
 // registers; the partials meet in shared memory and are summed over the warps
 // in a fixed order by the threads that finish the tile's elements.
 // Shared memory: P, S coefficients (2 (mcap+1) elements) + 2 * warps * 32U elements.
-template <typename CV, int U>
-__global__ void __launch_bounds__(AX2_THREADS) k_axpy2s(CV *__restrict__ V, long long n, KrylovPtrs kp) {
+// MINB blocks per SM: 3 (FP64) or 4 where the tiles outnumber two per SM.
+template <typename CV, int U, int MINB = 1>
+__global__ void __launch_bounds__(AX2_THREADS, MINB) k_axpy2s(CV *__restrict__ V, long long n, KrylovPtrs kp) {
     kp = kp_sys(kp);  // this block's system of a bucket
     V = sys_vec(V, kp);
     typedef typename real_of<CV>::type R;
@@ -878,11 +881,13 @@ __global__ void __launch_bounds__(AX2_THREADS) k_axpy2(CV *__restrict__ V, long 
 // group-major k_dots2, 5, 6 = tile-major k_dots2t with U = 4, 8, 7, 8 = split
 // k_dots2s with U = 8, 4, 9 = tile-major with U = 16 for FP32 (8 for FP64),
 // 10 = tile-major with U = 14 for FP32 (7 for FP64), 11, 12 = FP32 tile-major
-// on 16-byte pairs (float4 loads) with 16, 14 points per lane (even n; FP64: 6, 10).
+// on 16-byte pairs (float4 loads) with 16, 14 points per lane (even n; FP64: 6, 10),
+// 13 = 7 with two blocks per SM.
 // Axpy pass: 0-2 = j-unroll 4, 2, 8 of the element-major k_axpy2, 3, 4 =
 // tile-major k_axpy2t with U = 4, 8, 5, 6 = split k_axpy2s with U = 4, 2,
 // 7, 8 = tile-major with U = 16, 14 for FP32 (8, 7 for FP64), 9, 10 = FP32
-// tile-major on 16-byte pairs with 8, 14 points per lane (even n; FP64: 4, 8).
+// tile-major on 16-byte pairs with 8, 14 points per lane (even n; FP64: 4, 8),
+// 11 = 5 with three (FP64) or four blocks per SM.
 // Measured on B200:
 //   N = 1024, restart 100 (300 steps, k = 0..99), ms per 300 steps:
 //     FP64 dots 91.6 (shape 0), 81.0 (4), 59.4 (5), 54.3 (6, 4.9 TB/s)
@@ -894,7 +899,11 @@ __global__ void __launch_bounds__(AX2_THREADS) k_axpy2(CV *__restrict__ V, long 
 //     96 x 96 GMRES(200) FP64 (180 steps) 30.6 / 18.9 / 27.9 ms
 //     512 x 512 GMRES(200) FP64 (1000 steps) 0.381 / 0.254 / 0.327 s
 // Defaults: tile-major on grids with tile_major(n), widths by balanced(),
-// split (7, 5) below.
+// split below: (13, 11), whose blocks leave an SM room for two (three or four), where
+// the tiles outnumber the SMs, else (7, 5), which keep their registers.  Measured, us
+// per step over 100 steps, (7, 5) / (13, 11): FP64 256^2 50.0 / 47.7, 400^2 98.7 /
+// 88.5, 512^2 126.5 / 116.0; complex64 cycles 512^2 78.6 / 77.2; on 64^2, where
+// every tile has an SM of its own, 32.4 / 33.1.
 // CUGMRES_DOTS2_SHAPE / CUGMRES_AXPY2_SHAPE override them (diagnostics).
 static int env_shape(const char *name, int nshapes) {
     const char *e = getenv(name);
@@ -928,16 +937,16 @@ static int balanced(long long n, int sms, int va, int Ua, int vb, int Ub) {
     return cost(Ub) < cost(Ua) ? vb : va;
 }
 static int dots2_shape(int prec_v, long long n, int sms) {
-    static const int v = env_shape("CUGMRES_DOTS2_SHAPE", 13);
+    static const int v = env_shape("CUGMRES_DOTS2_SHAPE", 14);
     if (v >= 0) return v;
-    if (!tile_major(n, sms)) return 7;
+    if (!tile_major(n, sms)) return n > 256LL * sms ? 13 : 7;
     if (prec_v == 0) return balanced(n, sms, 6, 8, 10, 7);
     return n % 2 == 0 ? balanced(n, sms, 11, 16, 12, 14) : balanced(n, sms, 9, 16, 10, 14);
 }
 static int axpy2_shape(int prec_v, long long n, int sms) {
-    static const int v = env_shape("CUGMRES_AXPY2_SHAPE", 11);
+    static const int v = env_shape("CUGMRES_AXPY2_SHAPE", 12);
     if (v >= 0) return v;
-    if (!tile_major(n, sms)) return 5;
+    if (!tile_major(n, sms)) return n > 128LL * 2 * sms ? 11 : 5;
     if (prec_v == 0) return balanced(n, sms, 4, 8, 8, 7);
     return n % 2 == 0 ? balanced(n, sms, 9, 8, 10, 14) : balanced(n, sms, 4, 8, 8, 14);
 }
@@ -968,6 +977,7 @@ template <typename CV, bool COMP> struct Dots2Table {
             case 12:
                 if constexpr (sizeof(CV) == 8) return k_dots2t<CV, 14>;
                 else return k_dots2t<CV, 7>;
+            case 13: return k_dots2s<CV, 8, 2>;
             default: return k_dots2<CV, COMP, 4, 2>;
         }
     }
@@ -981,6 +991,7 @@ template <typename CV> struct Axpy2Table {
             case 3: return k_axpy2t<CV, 4>;
             case 4: return k_axpy2t<CV, 8>;
             case 5: return k_axpy2s<CV, 4>;
+            case 11: return k_axpy2s<CV, 4, sizeof(CV) == 16 ? 3 : 4>;
             case 6: return k_axpy2s<CV, 2>;
             case 7:  // 16 points per lane for FP32 vectors
                 if constexpr (sizeof(CV) == 8) return k_axpy2t<CV, 16>;
@@ -1004,7 +1015,7 @@ template <typename CV> struct Axpy2Table {
 static size_t dots2_smem(int v, int mcap) {
     const int jc = mcap + 1 < D2T_CHUNK ? mcap + 1 : D2T_CHUNK;
     if (v == 5 || v == 6 || (v >= 9 && v <= 12)) return (size_t)D2_WARPS * (size_t)jc * 4 * sizeof(double);
-    if (v == 7 || v == 8) return (size_t)jc * 4 * sizeof(double);
+    if (v == 7 || v == 8 || v == 13) return (size_t)jc * 4 * sizeof(double);
     return 0;
 }
 
@@ -1044,12 +1055,12 @@ int dots2_blocks(int prec_v, int sms, int mcap, long long n) {
     int g = dots2_vec(prec_v, n, v) ? waves_grid(dots2_vec_kernel(v, smem), D2_THREADS, smem, sms)
             : prec_v == 0           ? waves_grid(dots2_kernel<double2, false>(v, smem), D2_THREADS, smem, sms)
                                     : waves_grid(dots2_kernel<float2, true>(v, smem), D2_THREADS, smem, sms);
-    if (v >= 5 && v <= 12) {
+    if (v >= 5) {
         // points per lane, in complex values
         const int U = (v == 5 || v == 8) ? 4
                       : (v == 10 || v == 12) ? (prec_v != 0 ? 14 : 7)
                       : ((v == 9 || v == 11) && prec_v != 0) ? 16 : 8;
-        const long long cap = work_blocks(v == 7 || v == 8, U, n);
+        const long long cap = work_blocks(v == 7 || v == 8 || v == 13, U, n);
         if (cap < g) g = (int)cap;
     }
     return g;
@@ -1088,7 +1099,7 @@ template <typename CV> static int axpy2_prepare(int v, size_t smem) {
 static size_t axpy2_smem(int v, int prec_v, int mcap) {
     const size_t e = prec_v == 0 ? sizeof(double2) : sizeof(float2);
     size_t b = 2 * (size_t)(mcap + 1) * e;
-    if (v == 5 || v == 6) b += 2 * (size_t)(AX2_THREADS / 32) * 32 * (v == 5 ? 4 : 2) * e;
+    if (v == 5 || v == 6 || v == 11) b += 2 * (size_t)(AX2_THREADS / 32) * 32 * (v == 6 ? 2 : 4) * e;
     return b;
 }
 
@@ -1105,14 +1116,14 @@ int axpy2_blocks(int prec_v, int sms, int mcap, long long n) {
         axpy2_prepare<float2>(v, smem);
         g = waves_grid(Axpy2Table<float2>::get(v), AX2_THREADS, smem, sms);
     }
-    if (v >= 3 && v <= 10) {
+    if (v >= 3) {
         // points per lane, in complex values
-        const int U = (v == 3 || v == 5) ? 4
+        const int U = (v == 3 || v == 5 || v == 11) ? 4
                       : (v == 4 || v == 9) ? 8
                       : v == 6 ? 2
                       : (v == 8 || v == 10) ? (prec_v != 0 ? 14 : 7)
                                             : (prec_v != 0 ? 16 : 8);
-        const long long cap = work_blocks(v == 5 || v == 6, U, n);
+        const long long cap = work_blocks(v == 5 || v == 6 || v == 11, U, n);
         if (cap < g) g = (int)cap;
     }
     return g;
