@@ -33,6 +33,7 @@
 #include "cg_fft.cuh"
 #include "cg_fno.h"
 #include "cg_internal.h"
+#include "cg_wfft.cuh"
 
 using namespace cg;
 
@@ -85,7 +86,7 @@ struct cg_ctx {
     // two slots: a design loop alternates solves with A and with A^T
     struct CycleGraph {
         cudaGraphExec_t exec = nullptr;
-        unsigned char key[256] = {0};
+        unsigned char key[320] = {0};
         unsigned long long used = 0;
     } graphs[2];
     unsigned long long graph_clock = 0;
@@ -174,6 +175,10 @@ int next_embedding(int N) {
     while (L < 2 * N - 1) L *= 2;
     return L;
 }
+
+// entries of the twiddle tables: 4 L of cg_fft.cuh, then those of cg_wfft.cuh,
+// which the embedding of the one-kernel cycles uses
+size_t tw_entries(int L) { return 4 * (size_t)L + (L == 128 ? wtw_entries(wplan_r1(L / 2)) : 0); }
 
 double now_s() {
     timespec t;
@@ -528,6 +533,11 @@ int autotune(cg_ctx *c, int prec) {
 int apply_explicit(cg_ctx *c, int prec, int mode, int out_prec, const void *x, const void *b, void *y, double *npart,
                    int transpose = 0) {
     MatvecArgs a = margs(c, prec, transpose);
+    // one launch of a cluster where three kernels would each wait for the last one's few microseconds
+    if (mode == 0 && !npart && x != y && small_cycle_fits(prec, c->N, c->L, 0)) {
+        CG_LAUNCH(launch_small_matvec(prec, x, y, a, c->stream));
+        return CG_OK;
+    }
     CG_LAUNCH(launch_rows_forward(prec, a, fixed_vec(x), nullptr, nullptr, GATE_NONE, c->stream));
     CG_LAUNCH(launch_cols_convolve(prec, a, nullptr, GATE_NONE, c->stream));
     CG_LAUNCH(launch_rows_inverse(prec, mode, out_prec, a, fixed_vec(x), nullptr, b, fixed_vec(y), npart, nullptr,
@@ -915,17 +925,19 @@ int cugmres_set_operator(cg_ctx *c, int N, const cg_c128 *g_block, const double 
         CG_CU(cudaMalloc((void **)&c->c64, sizeof(double) * n));
         CG_CU(cudaMalloc((void **)&c->c32, sizeof(float) * n));
         CG_CU(cudaMalloc((void **)&c->chi32, sizeof(float) * n));
-        CG_CU(cudaMalloc((void **)&c->tw64, sizeof(double2) * 4 * L));
-        CG_CU(cudaMalloc((void **)&c->tw32, sizeof(float2) * 4 * L));
+        CG_CU(cudaMalloc((void **)&c->tw64, sizeof(double2) * tw_entries(L)));
+        CG_CU(cudaMalloc((void **)&c->tw32, sizeof(float2) * tw_entries(L)));
         CG_CU(cudaMalloc(&c->T, sizeof(double2) * (size_t)N * L));
         CG_CU(cudaMalloc((void **)&c->bbuf, sizeof(double2) * n));
         CG_CU(cudaMalloc((void **)&c->xbuf, sizeof(double2) * n));
         CG_CU(cudaMalloc((void **)&c->rbuf, sizeof(double2) * n));
     }
     // per-stage twiddle tables (cg_fft.cuh layout) of the 16- and 8-point
-    // plans, forward exp(-2 pi i m / L) and inverse, computed in double
-    std::vector<double2> tw(4 * L);
-    std::vector<float2> twf(4 * L);
+    // plans, forward exp(-2 pi i m / L) and inverse, then the tables of the
+    // warp-level transforms (cg_wfft.cuh), all computed in double
+    const size_t ntw = tw_entries(L);
+    std::vector<double2> tw(ntw);
+    std::vector<float2> twf(ntw);
     const double pi = 3.14159265358979323846;
     for (int t = 0; t < 4; t++) {
         const double sg = (t & 1) ? 1.0 : -1.0;
@@ -935,9 +947,13 @@ int cugmres_set_operator(cg_ctx *c, int N, const cg_c128 *g_block, const double 
             tw[(size_t)t * L + i] = m < 0 ? make_double2(0.0, 0.0) : make_double2(cos(a), sg * sin(a));
         }
     }
+    for (size_t i = 4 * (size_t)L; i < ntw; i++) {
+        const double a = 2.0 * pi * (double)wtw_exponent(L, wplan_r1(L / 2), (int)(i - 4 * (size_t)L)) / (double)L;
+        tw[i] = make_double2(cos(a), -sin(a));
+    }
     for (size_t i = 0; i < tw.size(); i++) twf[i] = make_float2((float)tw[i].x, (float)tw[i].y);
-    CG_CU(cudaMemcpyAsync(c->tw64, tw.data(), sizeof(double2) * 4 * L, cudaMemcpyHostToDevice, c->stream));
-    CG_CU(cudaMemcpyAsync(c->tw32, twf.data(), sizeof(float2) * 4 * L, cudaMemcpyHostToDevice, c->stream));
+    CG_CU(cudaMemcpyAsync(c->tw64, tw.data(), sizeof(double2) * ntw, cudaMemcpyHostToDevice, c->stream));
+    CG_CU(cudaMemcpyAsync(c->tw32, twf.data(), sizeof(float2) * ntw, cudaMemcpyHostToDevice, c->stream));
     double2 *g_tmp = nullptr;
     double *chi_tmp = nullptr;
     const double2 *gp = (const double2 *)g_block;
@@ -1249,7 +1265,14 @@ int cugmres_solve(cg_ctx *c, const cg_c128 *b, cg_c128 *x, const cg_opts *opts_i
     // One restart cycle: `steps` Arnoldi steps (launches after the device
     // stops the cycle return at once), back-solve and solution update.
     bool use_prec = learned;  // this cycle runs the learned preconditioner
+    // small grids: the steps up to the device's stop as one kernel (profiled cycles
+    // keep their phases, flexible GMRES ends some cycles after a number of launches)
+    const bool small = want_delayed && !learned && !c->prof && small_cycle_fits(prec, c->N, c->L, c->mcap);
     auto enqueue_steps = [&](int steps, cudaStream_t q) -> int {
+        if (small) {
+            CG_LAUNCH(launch_small_cycle(prec, c->V, n, kp, ap, q));
+            return CG_OK;
+        }
         for (int i = 0; i < steps; i++) {
             if (delayed) {
                 // w = A u_k into V[k+1]; one dot pass; normalisation + Givens; one axpy pass
@@ -1425,12 +1448,12 @@ int cugmres_solve(cg_ctx *c, const cg_c128 *b, cg_c128 *x, const cg_opts *opts_i
     // changes between cycles (not while profiling, not with the network).
     // (flexible GMRES: plain cycles after the probe only)
     const bool graphs = !c->prof && !c->in_probe && graphs_enabled();
-    unsigned char key[256];
+    unsigned char key[320];
     // key of the cycle about to be replayed (the scheme can change between cycles)
     auto make_key = [&]() {
         memset(key, 0, sizeof(key));
         struct K {
-            int prec, delayed, m, transpose, ndot, nax, ndot2, nax2, nrb, mcap, var[2][3], ss, nss;
+            int prec, delayed, m, transpose, ndot, nax, ndot2, nax2, nrb, mcap, var[2][3], ss, nss, small;
             long long n;
             const void *V, *x, *b, *st, *scale, *part;
             double2 shifts[SS_MAX];
@@ -1441,6 +1464,7 @@ int cugmres_solve(cg_ctx *c, const cg_c128 *b, cg_c128 *x, const cg_opts *opts_i
         memcpy(kk.var, c->var, sizeof(kk.var));
         kk.V = c->V, kk.x = xp, kk.b = bp, kk.st = c->st, kk.scale = kp.scale, kk.part = kp.part;
         kk.ss = ss_on ? S : 0;
+        kk.small = small;
         kk.nss = nss;
         if (ss_on) memcpy(kk.shifts, shifts, sizeof(shifts));
         static_assert(sizeof(K) <= sizeof(key), "graph key");
@@ -1456,7 +1480,7 @@ int cugmres_solve(cg_ctx *c, const cg_c128 *b, cg_c128 *x, const cg_opts *opts_i
             if (slot->exec) cudaGraphExecDestroy(slot->exec);
             slot->exec = nullptr;
             if (!c->cap_stream) CG_CU(cudaStreamCreateWithFlags(&c->cap_stream, cudaStreamNonBlocking));
-            if (!ss_on) {
+            if (!ss_on && !small) {
                 CG_TRY(cycle_graph(
                     kp, c->cap_stream, [&](cudaStream_t q) { return enqueue_steps(LOOP_STEPS, q); },
                     [&](cudaStream_t q) -> int {
@@ -1467,7 +1491,7 @@ int cugmres_solve(cg_ctx *c, const cg_c128 *b, cg_c128 *x, const cg_opts *opts_i
             } else {
                 cudaGraph_t g = nullptr;
                 CG_CU(cudaStreamBeginCapture(c->cap_stream, cudaStreamCaptureModeThreadLocal));
-                int e1 = enqueue_cycle_ss(c->cap_stream, 0, ss_nblk, true);
+                int e1 = ss_on ? enqueue_cycle_ss(c->cap_stream, 0, ss_nblk, true) : enqueue_cycle(1, c->cap_stream);
                 int e2 = e1 == CG_OK ? enqueue_begin(c->cap_stream) : e1;
                 cudaError_t ce = cudaStreamEndCapture(c->cap_stream, &g);
                 if (e2 != CG_OK || ce != cudaSuccess) {

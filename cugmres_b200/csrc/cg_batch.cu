@@ -374,7 +374,12 @@ int solve_bucket(cg_ctx *ctx, const cg_system *sys, const std::vector<int> &idx,
         BK_LAUNCH(launch_cycle_begin(kp, nrb, q));
         return CG_OK;
     };
+    const bool small = small_cycle_fits(prec, N, L, m);  // a cluster per system runs its whole cycle
     auto enqueue_steps = [&](cudaStream_t q) -> int {
+        if (small) {
+            BK_LAUNCH(launch_small_cycle(prec, bb.V, n, kp, ap, q));
+            return CG_OK;
+        }
         for (int i = 0; i < LOOP_STEPS; i++) {
             BK_LAUNCH(launch_rows_forward(prec, ap, vk, nullptr, kp.st, GATE_STOP, q));
             BK_LAUNCH(launch_cols_convolve(prec, ap, kp.st, GATE_STOP, q));
