@@ -1337,11 +1337,12 @@ int cugmres_solve(cg_ctx *c, const cg_c128 *b, cg_c128 *x, const cg_opts *opts_i
     // block's later vectors kept almost nothing outside the basis, so its
     // Cholesky failed and the cycle restarted (512^2, eps_r = 4, restart 4500:
     // 7 cycles and 12 000 steps without reaching 1e-10).  With the refresh the
-    // first cycle runs 3981 steps (delayed CGS2: 3979) and a second of 1663
-    // removes the 1e-8 its Hessenberg reconstruction left.  Each cycle starts
+    // first cycle runs 3981 steps (delayed CGS2: 3979) and a second of 1420 to
+    // 1670 removes the 1e-8 its Hessenberg reconstruction left.  Each cycle starts
     // again from the probe's shifts.
     constexpr int SS_REFRESH_MIN = 256, SS_REFRESH_STEPS = 100, SS_REFRESH_WINDOW = 32;
     const bool ss_segments = m > SS_REFRESH_MIN;
+    kp.ss_tau = ss_segments ? SS_ONE_PASS_LONG : SS_ONE_PASS;
     const int ss_nblk = S > 0 ? (m + S - 1) / S : 0;  // blocks of a full s-step cycle
     double2 shifts0[SS_MAX];
     for (int i = 0; i < SS_MAX; i++) shifts0[i] = make_double2(0.0, 0.0);

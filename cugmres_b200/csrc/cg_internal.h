@@ -53,7 +53,7 @@ struct DevState {
     double2 du;       //   u_{k+1} = cw w + du u - sum S_j q_j
     double2 delta;    // q_k^H w of the current delayed CGS2 step
     unsigned int counter[8];  // tickets of the last-block reductions
-    int ss_one;               // s-step: the block's first Gram-Schmidt pass was enough (second pass skipped)
+    int ss_one;               // s-step: 1: the block's first Gram-Schmidt pass was enough (second pass skipped)
 };
 
 // Device workspace of one Krylov cycle (restart m, budget maxit).
@@ -79,6 +79,7 @@ struct KrylovPtrs {
     double *gpart;   // [ceil(nblk_dots2 / 16) * 4 * part_ld] group sums of the dot partials
     unsigned int *tickets;  // [ceil(nblk_dots2 / 16)] arrival counters of those groups (reset by the last)
     double2 *ss = nullptr;  // s-step scratch (cg_sstep.cu: block coefficients, Gram, shifts, work rows)
+    double ss_tau = 0.0;    // s-step, FP64: threshold of the one-pass blocks (SS_ONE_PASS)
     int mcap;        // allocated restart capacity (leading dimension of Rm / part)
     // Bucket of systems solved in lockstep (one launch covers all of them,
     // system = blockIdx.y): every array above (st included) of system s lies
@@ -213,6 +214,20 @@ int launch_small_matvec(int prec, const void *x, void *y, const MatvecArgs &a, c
 int launch_small_cycle(int prec, void *V, long long n, const KrylovPtrs &kp, const MatvecArgs &a, cudaStream_t s);
 // s-step Arnoldi (cg_sstep.cu): S steps per block, S in {2, 4, 8}
 constexpr int SS_MAX = 8;
+// An FP64 block whose first pass keeps more than this fraction of every
+// vector's squared norm skips the second pass: the first pass then leaves the
+// block orthogonal to about eps / fraction (2e-15).  Measured: the 1024^2
+// GMRES(100) blocks keep 0.1 to 0.3, and the 64^2 solves keep their step counts
+// (699, 699, 673 with S = 2, 4, 8), which a 1e-2 threshold did not (711 with S = 2).
+// Complex64 blocks always take both passes (eps = 6e-8).
+constexpr double SS_ONE_PASS = 0.1;
+// ... and this in a long (segmented) cycle, where the loss of the first blocks
+// grows over thousands of steps until a later block's Cholesky fails and the
+// restart throws the Krylov space away.  512^2, eps_r = 4, restart 4500, to
+// 1e-10 with five sets of FFT launch shapes, which differ in rounding only: at
+// 0.1 7457, 7779, 6953, 5379 and 9000 steps (the last without converging), 7.5 to
+// 9.5 s; at 0.5 5404, 5449, 5519, 5651 and 5558, 7.5 to 7.9 s.
+constexpr double SS_ONE_PASS_LONG = 0.5;
 int sstep_supported(int S);
 long long sstep_scratch_elems(int mcap);  // double2 entries of KrylovPtrs::ss
 int sstep_part_ld(int mcap);              // partials per block of the block dot pass

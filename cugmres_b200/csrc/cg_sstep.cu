@@ -50,13 +50,6 @@ template <typename CV> constexpr int ss_minb() { return sizeof(CV) == 16 ? 1 : 2
 // stages of a warp's private basis-tile ring in the dot pass (cp.async, one
 // commit group per basis vector, each lane copying and reading its own points)
 static constexpr int SS_NST = 4;
-// An FP64 block whose first pass keeps more than this fraction of every
-// vector's squared norm skips the second pass: the first pass then leaves the
-// block orthogonal to about eps / fraction (2e-15).  Measured: the 1024^2
-// GMRES(100) blocks keep 0.1 to 0.3, and the 64^2 solves keep their step counts
-// (699, 699, 673 with S = 2, 4, 8), which a 1e-2 threshold did not (711 with S = 2).
-// Complex64 blocks always take both passes (eps = 6e-8).
-static constexpr double SS_ONE_PASS = 0.1;
 
 static __device__ __forceinline__ void cp_async_cv(double2 *dst, const double2 *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
@@ -455,7 +448,7 @@ __global__ void __launch_bounds__(SS_THREADS, ss_minb<CV>()) k_ss_dots(const CV 
     }
     // the last block goes on with the pass's Cholesky (C and G are complete)
     __syncthreads();
-    ss_chol<S>(kp, pass, sizeof(CV) == 16 ? SS_ONE_PASS : 2.0);  // q <= 1: complex64 never skips
+    ss_chol<S>(kp, pass, sizeof(CV) == 16 ? kp.ss_tau : 2.0);  // q <= 1: complex64 never skips
 }
 
 // ------------------------------------------------------------ update
