@@ -113,7 +113,7 @@ struct MatvecArgs {
     const void *gq;     // quarter spectrum (C)
     const void *cdiag;  // N x N real diagonal k0^2 chi (R)
     const void *tw;     // L twiddles (C)
-    void *T;            // N x L intermediate (C)
+    void *T;            // N x L intermediate (C), columns in groups (cg_tlayout.cuh)
     int transpose = 0;  // 1: A^T x = x - diag(c) G x (contrast applied after the convolution)
     int sms = 148;      // multiprocessors of the device (grid of the persistent column pass)
     int nsys = 1;       // systems of a bucket (grid.y of every pass)

@@ -8,7 +8,8 @@
 //
 // Here:
 //   pass 1  k_rows_forward   rows 0..N-1 only: load x and c, scale, zero-pad in
-//                            registers, forward row FFT, store T[N][L].
+//                            registers, forward row FFT, store N x L values T
+//                            (columns in groups, cg_tlayout.cuh).
 //   pass 2  k_cols_convolve  per column: forward column FFT (upper half of the
 //                            input is zero), multiply by the spectrum, inverse
 //                            column FFT, store only rows 0..N-1 back into T.
@@ -30,6 +31,7 @@
 // per (precision, L); smaller L always use variant 0.
 #include "cg_fft.cuh"
 #include "cg_internal.h"
+#include "cg_tlayout.cuh"
 
 namespace cg {
 
@@ -58,10 +60,10 @@ typedef MvShape<16, 256, 256, 512, 1, 1> MvV5;  // V0 with the pipelined column 
 typedef MvShape<8, 256, 512, 512, 1, 1> MvV6;   // V2 with the pipelined column pass
 // 16 points, smaller column blocks, two per SM (each block's barriers hold
 // only its own warps, so one block's shared-memory exchanges can overlap the
-// other's butterflies).  Measured at L = 2048 (ncu): FP32 column pass 30.3 us
-// against 32.6 us for V0 (two columns per 256-thread block); FP64 60.6 us
-// against 53.4 us (one column per 128-thread block: its loads use 16 of each
-// 32-byte sector of T).
+// other's butterflies).  Measured at L = 2048 (ncu, warm L2): FP32 column pass 23.9
+// us against 28.7 us for V1 (four columns per 512-thread block); FP64 44.2 us
+// against 43.5 us for V1 (one column per 128-thread block: its loads use 16 of
+// each 32-byte sector of T).
 typedef MvShape<16, 256, 128, 256, 2> MvV7;
 // V0's transforms with the grouped pipelined column pass (k_cols_convolve_grp):
 // each column transform of a block is an independent worker with its own
@@ -129,9 +131,9 @@ k_rows_forward(VecSel xs, const double *__restrict__ xscale, const typename real
     }
     fft_run<L, SH::E, false, true>(reg, sm, tw, t);
     if (live) {
-        C *out = T + (size_t)row * L;
+        C *out = T + (size_t)row * t_group<C>();
 #pragma unroll
-        for (int p = 0; p < E; p++) out[t + p * TPR] = reg[p];
+        for (int p = 0; p < E; p++) out[t_column<C>(t + p * TPR, N)] = reg[p];
     }
 }
 
@@ -155,12 +157,13 @@ k_cols_convolve(C *__restrict__ T, const C *__restrict__ gq, const C *__restrict
     const int b = blockIdx.x;
     const int tile = (b & 1) ? (ntiles - 1 - (b >> 1)) : (b >> 1);
     const int col = tile * CPB + cl;
+    C *tc = T + t_column<C>(col, N);
     C reg[E];
 #pragma unroll
     for (int p = 0; p < E; p++) {
         const int k = t + p * TPR;
         reg[p] = czero<C>();
-        if (p < E / 2 && k < N) reg[p] = T[(size_t)k * L + col];
+        if (p < E / 2 && k < N) reg[p] = tc[(size_t)k * t_group<C>()];
     }
     fft_run<L, SH::E, false, true, CPB>(reg, sm, tw, t);
     const int Lq = L / 2 + 1;
@@ -175,7 +178,7 @@ k_cols_convolve(C *__restrict__ T, const C *__restrict__ gq, const C *__restrict
 #pragma unroll
     for (int p = 0; p < E / 2; p++) {
         const int k = t + p * TPR;
-        if (k < N) T[(size_t)k * L + col] = reg[p];
+        if (k < N) tc[(size_t)k * t_group<C>()] = reg[p];
     }
 }
 
@@ -243,7 +246,7 @@ k_cols_convolve_pipe(C *__restrict__ T, const C *__restrict__ gq, const C *__res
         C *gd = td + G::TD;
         const int col0 = tile_of(v) * CPB;
         for (int e = threadIdx.x; e < N * CPB; e += THREADS)
-            cp_async_elem(td + e, T + (size_t)(e / CPB) * L + col0 + (e % CPB));
+            cp_async_elem(td + e, T + t_column<C>(col0 + e % CPB, N) + (size_t)(e / CPB) * t_group<C>());
         for (int e = threadIdx.x; e < LQ * CPB; e += THREADS) {
             const int c = e / LQ, qr = e % LQ;
             const int col = col0 + c;
@@ -265,7 +268,7 @@ k_cols_convolve_pipe(C *__restrict__ T, const C *__restrict__ gq, const C *__res
         __syncthreads();
         const C *td = buf + slot * G::SLOT;
         const C *gd = td + G::TD;
-        const int col = tile_of(v) * CPB + cl;
+        C *tc = T + t_column<C>(tile_of(v) * CPB + cl, N);
         C reg[E];
 #pragma unroll
         for (int p = 0; p < E; p++) {
@@ -284,7 +287,7 @@ k_cols_convolve_pipe(C *__restrict__ T, const C *__restrict__ gq, const C *__res
 #pragma unroll
         for (int p = 0; p < E / 2; p++) {
             const int k = t + p * TPR;
-            if (k < N) T[(size_t)k * L + col] = reg[p];
+            if (k < N) tc[(size_t)k * t_group<C>()] = reg[p];
         }
         __syncthreads();  // this slot is refilled by the next iteration's issue
     }
@@ -335,7 +338,8 @@ k_cols_convolve_grp(C *__restrict__ T, const C *__restrict__ gq, const C *__rest
     auto issue = [&](int col, int slot) {
         C *td = buf + slot * G::SLOT;
         C *gd = td + G::TD;
-        for (int e = t; e < N; e += TPR) cp_async_elem(td + e, T + (size_t)e * L + col);
+        const C *tc = T + t_column<C>(col, N);
+        for (int e = t; e < N; e += TPR) cp_async_elem(td + e, tc + (size_t)e * t_group<C>());
         const int qc = col <= L / 2 ? col : L - col;
         for (int e = t; e < LQ; e += TPR) cp_async_elem(gd + e, gq + (size_t)qc * LQ + e);
         cp_async_commit();
@@ -370,7 +374,7 @@ k_cols_convolve_grp(C *__restrict__ T, const C *__restrict__ gq, const C *__rest
 #pragma unroll
         for (int p = 0; p < E / 2; p++) {
             const int k = t + p * TPR;
-            if (k < N) T[(size_t)k * L + col] = reg[p];
+            if (k < N) T[t_column<C>(col, N) + (size_t)k * t_group<C>()] = reg[p];
         }
         fft_barrier<NT>(bar);  // this slot is refilled by the next iteration's issue
     }
@@ -453,9 +457,9 @@ k_rows_forward_pipe(VecSel xs, const double *__restrict__ xscale, const typename
             }
         }
         fft_run_wb<L, SH::E, false, true, 1, NT>(reg, sm, wb, t, bar);
-        C *out = T + (size_t)row * L;
+        C *out = T + (size_t)row * t_group<C>();
 #pragma unroll
-        for (int p = 0; p < E; p++) out[t + p * TPR] = reg[p];
+        for (int p = 0; p < E; p++) out[t_column<C>(t + p * TPR, N)] = reg[p];
         fft_barrier<NT>(bar);  // this slot is refilled by the next iteration's issue
     }
     cp_async_wait<0>();
@@ -503,9 +507,9 @@ k_rows_inverse(const C *__restrict__ T, VecSel xs, const double *__restrict__ xs
         bv[p] = (MODE != 0 && ok) ? bvec[rb + idx] : czero<C>();
     }
     if (live) {
-        const C *in = T + (size_t)row * L;
+        const C *in = T + (size_t)row * t_group<C>();
 #pragma unroll
-        for (int p = 0; p < E; p++) reg[p] = in[t + p * TPR];
+        for (int p = 0; p < E; p++) reg[p] = in[t_column<C>(t + p * TPR, N)];
     } else {
 #pragma unroll
         for (int p = 0; p < E; p++) reg[p] = czero<C>();
@@ -584,10 +588,10 @@ k_rows_inv_fwd(C *__restrict__ T, VecSel xs, VecSel ys, const typename real_of<C
         xv[p] = ok ? x[rb + idx] : czero<C>();
         cv[p] = ok ? cdiag[rb + idx] : (R)0;
     }
-    C *trow = T + (size_t)row * L;
+    C *trow = T + (size_t)row * t_group<C>();
     if (live) {
 #pragma unroll
-        for (int p = 0; p < E; p++) reg[p] = trow[t + p * TPR];
+        for (int p = 0; p < E; p++) reg[p] = trow[t_column<C>(t + p * TPR, N)];
     } else {
 #pragma unroll
         for (int p = 0; p < E; p++) reg[p] = czero<C>();
@@ -609,7 +613,7 @@ k_rows_inv_fwd(C *__restrict__ T, VecSel xs, VecSel ys, const typename real_of<C
     fft_run<L, SH::E, false, true>(reg, sm, tw, t);
     if (live) {
 #pragma unroll
-        for (int p = 0; p < E; p++) trow[t + p * TPR] = reg[p];
+        for (int p = 0; p < E; p++) trow[t_column<C>(t + p * TPR, N)] = reg[p];
     }
 }
 
