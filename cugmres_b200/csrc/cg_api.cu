@@ -72,6 +72,10 @@ struct cg_ctx {
     // autotuner leaves out the persistent column pass, which would hold every
     // SM's shared memory while the other streams' kernels wait
     bool shared_gpu = false;
+    void *oparena = nullptr;  // the operator's arrays (alloc_operator)
+    size_t oparena_cap = 0;
+    void *scratch = nullptr;  // temporaries of set_operator; contexts of a sweep keep them
+    size_t scratch_cap = 0;
     char devname[256] = {0};
     // per-phase timing
     bool prof = false;
@@ -102,6 +106,9 @@ struct cg_ctx {
 };
 
 namespace cg {
+// entries of the twiddle tables: 4 L of cg_fft.cuh, then those of cg_wfft.cuh,
+// which the embedding of the one-kernel cycles uses
+static size_t tw_entries(int L) { return 4 * (size_t)L + (L == 128 ? wtw_entries(wplan_r1(L / 2)) : 0); }
 void ctx_set_shared_gpu(cg_ctx *c, bool on) {
     if (c) c->shared_gpu = on;
 }
@@ -118,6 +125,7 @@ int ctx_op_view(const cg_ctx *c, OpView *v) {
     v->c32 = c->c32;
     v->tw64 = c->tw64;
     v->tw32 = c->tw32;
+    v->ntw = tw_entries(c->L);
     v->stream = c->stream;
     return CG_OK;
 }
@@ -176,10 +184,6 @@ int next_embedding(int N) {
     return L;
 }
 
-// entries of the twiddle tables: 4 L of cg_fft.cuh, then those of cg_wfft.cuh,
-// which the embedding of the one-kernel cycles uses
-size_t tw_entries(int L) { return 4 * (size_t)L + (L == 128 ? wtw_entries(wplan_r1(L / 2)) : 0); }
-
 double now_s() {
     timespec t;
     clock_gettime(CLOCK_MONOTONIC, &t);
@@ -235,19 +239,56 @@ int grid_for(long long n, int cap) {
     return (int)g;
 }
 
+// The operator's arrays lie in one allocation, the temporaries of its set-up in
+// another: eleven and three cudaMalloc / cudaFree pairs per operator took longer
+// than the set-up's kernels on sweeps of small grids (each free waits for the GPU).
 void free_operator(cg_ctx *c) {
-    dfree_t(c->gq64);
-    dfree_t(c->gq32);
-    dfree_t(c->c64);
-    dfree_t(c->c32);
-    dfree_t(c->chi32);
-    dfree_t(c->tw64);
-    dfree_t(c->tw32);
-    dfree(c->T);
-    dfree_t(c->bbuf);
-    dfree_t(c->xbuf);
-    dfree_t(c->rbuf);
+    dfree(c->oparena);
+    c->oparena_cap = 0;
+    c->gq64 = nullptr;
+    c->gq32 = nullptr;
+    c->c64 = nullptr;
+    c->c32 = c->chi32 = nullptr;
+    c->tw64 = nullptr;
+    c->tw32 = nullptr;
+    c->T = nullptr;
+    c->bbuf = c->xbuf = c->rbuf = nullptr;
     c->have_op = false;
+}
+
+void free_scratch(cg_ctx *c) {
+    dfree(c->scratch);
+    c->scratch_cap = 0;
+}
+
+// lays the operator's arrays out for c->N and c->L; a context of a sweep, which
+// takes its systems largest grid first, keeps an allocation that is large enough
+int alloc_operator(cg_ctx *c) {
+    const size_t L = c->L, n = (size_t)c->N * c->N, Lq = L / 2 + 1;
+    const size_t bytes[] = {sizeof(double2) * Lq * Lq, sizeof(float2) * Lq * Lq,  sizeof(double) * n,
+                            sizeof(float) * n,         sizeof(float) * n,         sizeof(double2) * tw_entries(c->L),
+                            sizeof(float2) * tw_entries(c->L), sizeof(double2) * c->N * L, sizeof(double2) * n,
+                            sizeof(double2) * n,       sizeof(double2) * n};
+    void **const ptr[] = {(void **)&c->gq64, (void **)&c->gq32, (void **)&c->c64,  (void **)&c->c32,
+                          (void **)&c->chi32, (void **)&c->tw64, (void **)&c->tw32, &c->T,
+                          (void **)&c->bbuf, (void **)&c->xbuf, (void **)&c->rbuf};
+    size_t total = 0;
+    for (size_t b : bytes) total += (b + 255) & ~(size_t)255;
+    if (!(c->shared_gpu && c->oparena && total <= c->oparena_cap)) {
+        free_operator(c);
+        if (int e = cuerr(cudaMalloc(&c->oparena, total))) {
+            cudaGetLastError();
+            c->oparena = nullptr;
+            return e;
+        }
+        c->oparena_cap = total;
+    }
+    char *at = (char *)c->oparena;
+    for (size_t i = 0; i < sizeof(bytes) / sizeof(bytes[0]); i++) {
+        *ptr[i] = at;
+        at += (bytes[i] + 255) & ~(size_t)255;
+    }
+    return CG_OK;
 }
 
 void free_graph(cg_ctx *c) {
@@ -814,6 +855,7 @@ int cugmres_destroy(cg_ctx *c) {
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     free_operator(c);
+    free_scratch(c);
     free_krylov(c);
     dfree_t(c->st);
     if (c->st_host) cudaFreeHost(c->st_host);
@@ -883,12 +925,10 @@ int cugmres_grid_size(const cg_ctx *c, int *N, int *L) {
     return CG_OK;
 }
 
-static int set_operator_dev(cg_ctx *c, int N, const double2 *g_dev, const double *chi_dev, double chi_scale) {
+static int set_operator_dev(cg_ctx *c, int N, const double2 *g_dev, const double *chi_dev, double chi_scale, double2 *full) {
     const int L = c->L;
     const long long n = (long long)N * N;
     // spectrum: even embedding, full FP64 2D transform, quarter with 1/L^2 folded in
-    double2 *full = nullptr;
-    CG_CU(cudaMalloc((void **)&full, sizeof(double2) * (size_t)L * L));
     k_embed<<<grid_for((long long)L * L, 8 * c->sms), 256, 0, c->stream>>>(g_dev, full, N, L);
     int e = launch_fft2d_full_fp64(L, full, c->tw64, c->stream);
     if (e == 0) {
@@ -897,40 +937,29 @@ static int set_operator_dev(cg_ctx *c, int N, const double2 *g_dev, const double
         k_scale_real<<<grid_for(n, 8 * c->sms), 256, 0, c->stream>>>(chi_dev, chi_scale, c->c64, c->c32, c->chi32, n);
     }
     cudaError_t ce = cudaStreamSynchronize(c->stream);
-    cudaFree(full);
     if (e != 0) return CG_ERR_CUDA;
     return cuerr(ce);
 }
 
-int cugmres_set_operator(cg_ctx *c, int N, const cg_c128 *g_block, const double *chi, double chi_scale) {
-    if (!c || !g_block || !chi || N < 1 || !isfinite(chi_scale)) return CG_ERR_INVALID;
+// The block is given, or Green's function `kind` with k0 and h (g_block null).
+static int set_operator_any(cg_ctx *c, int N, const cg_c128 *g_block, int kind, double k0, double h, const double *chi,
+                            double chi_scale) {
     const int L = next_embedding(N);
     if (!fft_supported(L)) return CG_ERR_NOT_IMPLEMENTED;
     CG_CU(cudaSetDevice(c->device));
     const long long n = (long long)N * N;
-    const bool g_dev = is_device_ptr(g_block), chi_dev = is_device_ptr(chi);
-    if (!g_dev && !all_finite((const double *)g_block, 2 * (size_t)n)) return CG_ERR_NONFINITE;
+    const bool g_dev = g_block && is_device_ptr(g_block), chi_dev = is_device_ptr(chi);
+    if (g_block && !g_dev && !all_finite((const double *)g_block, 2 * (size_t)n)) return CG_ERR_NONFINITE;
     if (!chi_dev && !all_finite(chi, (size_t)n)) return CG_ERR_NONFINITE;
     // a context keeps its buffers when the grid size does not change (batched sweeps)
     const bool same = c->gq64 != nullptr && c->N == N && c->L == L;
     c->have_op = false;
     if (!same) {
-        free_operator(c);
+        if (!c->shared_gpu) free_operator(c);
         free_krylov(c);
         c->N = N;
         c->L = L;
-        const int Lq = L / 2 + 1;
-        CG_CU(cudaMalloc((void **)&c->gq64, sizeof(double2) * (size_t)Lq * Lq));
-        CG_CU(cudaMalloc((void **)&c->gq32, sizeof(float2) * (size_t)Lq * Lq));
-        CG_CU(cudaMalloc((void **)&c->c64, sizeof(double) * n));
-        CG_CU(cudaMalloc((void **)&c->c32, sizeof(float) * n));
-        CG_CU(cudaMalloc((void **)&c->chi32, sizeof(float) * n));
-        CG_CU(cudaMalloc((void **)&c->tw64, sizeof(double2) * tw_entries(L)));
-        CG_CU(cudaMalloc((void **)&c->tw32, sizeof(float2) * tw_entries(L)));
-        CG_CU(cudaMalloc(&c->T, sizeof(double2) * (size_t)N * L));
-        CG_CU(cudaMalloc((void **)&c->bbuf, sizeof(double2) * n));
-        CG_CU(cudaMalloc((void **)&c->xbuf, sizeof(double2) * n));
-        CG_CU(cudaMalloc((void **)&c->rbuf, sizeof(double2) * n));
+        CG_TRY(alloc_operator(c));
     }
     // per-stage twiddle tables (cg_fft.cuh layout) of the 16- and 8-point
     // plans, forward exp(-2 pi i m / L) and inverse, then the tables of the
@@ -954,28 +983,46 @@ int cugmres_set_operator(cg_ctx *c, int N, const cg_c128 *g_block, const double 
     for (size_t i = 0; i < tw.size(); i++) twf[i] = make_float2((float)tw[i].x, (float)tw[i].y);
     CG_CU(cudaMemcpyAsync(c->tw64, tw.data(), sizeof(double2) * ntw, cudaMemcpyHostToDevice, c->stream));
     CG_CU(cudaMemcpyAsync(c->tw32, twf.data(), sizeof(float2) * ntw, cudaMemcpyHostToDevice, c->stream));
-    double2 *g_tmp = nullptr;
-    double *chi_tmp = nullptr;
-    const double2 *gp = (const double2 *)g_block;
-    const double *cp = chi;
-    if (!g_dev) {
-        CG_CU(cudaMalloc((void **)&g_tmp, sizeof(double2) * n));
-        CG_CU(cudaMemcpyAsync(g_tmp, g_block, sizeof(double2) * n, cudaMemcpyHostToDevice, c->stream));
-        gp = g_tmp;
+    // temporaries: the embedding, the block and the contrast where the caller's are not on the device
+    const size_t full_bytes = sizeof(double2) * (size_t)L * L;
+    const size_t g_bytes = g_dev ? 0 : (sizeof(double2) * n + 255) & ~(size_t)255;
+    const size_t bytes = full_bytes + g_bytes + (chi_dev ? 0 : sizeof(double) * n);
+    if (bytes > c->scratch_cap) {
+        free_scratch(c);
+        if (int e = cuerr(cudaMalloc(&c->scratch, bytes))) {
+            cudaGetLastError();
+            c->scratch = nullptr;
+            return e;
+        }
+        c->scratch_cap = bytes;
     }
-    if (!chi_dev) {
-        CG_CU(cudaMalloc((void **)&chi_tmp, sizeof(double) * n));
-        CG_CU(cudaMemcpyAsync(chi_tmp, chi, sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));
-        cp = chi_tmp;
+    double2 *full = (double2 *)c->scratch;
+    double2 *g_tmp = (double2 *)((char *)c->scratch + full_bytes);
+    double *chi_tmp = (double *)((char *)c->scratch + full_bytes + g_bytes);
+    const double2 *gp = g_dev ? (const double2 *)g_block : g_tmp;
+    const double *cp = chi_dev ? chi : chi_tmp;
+    int s = CG_OK;
+    if (!g_block)
+        s = launch_green_block(kind, N, k0, h, g_tmp, c->sms, c->stream) ? CG_ERR_CUDA : CG_OK;
+    else if (!g_dev)
+        s = cuerr(cudaMemcpyAsync(g_tmp, g_block, sizeof(double2) * n, cudaMemcpyHostToDevice, c->stream));
+    if (s == CG_OK && !chi_dev)
+        s = cuerr(cudaMemcpyAsync(chi_tmp, chi, sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));
+    if (s == CG_OK) s = set_operator_dev(c, N, gp, cp, chi_scale, full);
+    if (!c->shared_gpu || s != CG_OK) {
+        cudaStreamSynchronize(c->stream);
+        free_scratch(c);
     }
-    int s = set_operator_dev(c, N, gp, cp, chi_scale);
-    if (g_tmp) cudaFree(g_tmp);
-    if (chi_tmp) cudaFree(chi_tmp);
     if (s != CG_OK) return s;
     CG_TRY(autotune(c, 0));
     CG_TRY(autotune(c, 1));
     c->have_op = true;
     return CG_OK;
+}
+
+int cugmres_set_operator(cg_ctx *c, int N, const cg_c128 *g_block, const double *chi, double chi_scale) {
+    if (!c || !g_block || !chi || N < 1 || !isfinite(chi_scale)) return CG_ERR_INVALID;
+    return set_operator_any(c, N, g_block, 0, 0.0, 0.0, chi, chi_scale);
 }
 
 static int green_args_ok(int kind, int N, double k0, double h) {
@@ -998,14 +1045,7 @@ int cugmres_green_block_device(int kind, int N, double k0, double h, cg_c128 *ou
 
 int cugmres_set_operator_green(cg_ctx *c, int kind, int N, double k0, double h, const double *chi, double chi_scale) {
     if (!c || !chi || !green_args_ok(kind, N, k0, h) || !isfinite(chi_scale)) return CG_ERR_INVALID;
-    CG_CU(cudaSetDevice(c->device));
-    double2 *g = nullptr;
-    CG_CU(cudaMalloc((void **)&g, sizeof(double2) * (size_t)N * N));
-    int st = launch_green_block(kind, N, k0, h, g, c->sms, c->stream) ? CG_ERR_CUDA : CG_OK;
-    if (st == CG_OK) st = cugmres_set_operator(c, N, (const cg_c128 *)g, chi, chi_scale);
-    cudaStreamSynchronize(c->stream);
-    cudaFree(g);
-    return st;
+    return set_operator_any(c, N, nullptr, kind, k0, h, chi, chi_scale);
 }
 
 int cugmres_set_operator_circulant(cg_ctx *c, int N, const cg_c64 *g_prep, const double *chi, double chi_scale) {

@@ -22,6 +22,7 @@
 #include <cmath>
 #include <functional>
 #include <map>
+#include <memory>
 #include <thread>
 #include <vector>
 
@@ -99,7 +100,8 @@ extern "C" int cugmres_solve_batch(int device, int nsys, const cg_system *sys, c
 // every later launch of its bucket; the restart cycle (delayed CGS2 steps while
 // a system runs, back-solve, update, the next true residual and cycle decisions
 // of all systems) is captured once per bucket as a CUDA graph and replayed
-// with one launch per cycle, one host synchronisation per cycle.
+// with one launch per cycle, one host synchronisation per cycle.  The buckets
+// of a sweep run side by side, each on its own stream (run_wave).
 // Scope: FP64 or mixed precision (complex64 cycles, FP64 residual and
 // update), delayed CGS2, no preconditioner, A x = b (not the transposed
 // system), restarted semantics; other options return CG_ERR_NOT_IMPLEMENTED.
@@ -164,19 +166,21 @@ WsLayout ws_layout(int mc, int maxit, size_t npart, size_t part, size_t gpart, s
     return w;
 }
 
+// One allocation holds a bucket's arrays (seven to eleven pairs of cudaMalloc and
+// cudaFree a bucket took longer than the cycles of small grids).
 struct BucketBufs {
+    void *all = nullptr;
     void *V = nullptr, *T = nullptr, *G = nullptr, *C = nullptr, *G32 = nullptr, *C32 = nullptr, *X = nullptr,
-         *B = nullptr, *WS = nullptr;
-    DevState *st_host = nullptr;
-    cudaStream_t cap = nullptr;
+         *B = nullptr, *WS = nullptr, *TW = nullptr, *TW32 = nullptr;
+    DevState *st_host = nullptr;  // the bucket's part of the sweep's pinned states
+    cudaStream_t run = nullptr;
     cudaGraphExec_t gexec = nullptr;
     cudaEvent_t ev = nullptr;
     ~BucketBufs() {
+        if (run) cudaStreamSynchronize(run);
         if (gexec) cudaGraphExecDestroy(gexec);
-        for (void *p : {V, T, G, C, G32, C32, X, B, WS})
-            if (p) cudaFree(p);
-        if (st_host) cudaFreeHost(st_host);
-        if (cap) cudaStreamDestroy(cap);
+        if (all) cudaFree(all);
+        if (run) cudaStreamDestroy(run);
         if (ev) cudaEventDestroy(ev);
     }
 };
@@ -208,16 +212,76 @@ bool on_device(const void *p) {
     return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
-// Solves the systems idx[0..B) (all of side N) as one bucket on ctx's device.
-int solve_bucket(cg_ctx *ctx, const cg_system *sys, const std::vector<int> &idx, const cg_opts &o, double t_sweep,
-                 cg_result *results) {
+// A bucket between its set-up and its results.
+struct Bucket {
+    BucketBufs bb;
+    std::vector<int> idx;  // its systems, all of one grid side
+    OpView ov{};
+    size_t gq_elems = 0;
+    int ndot2 = 0, nax2 = 0, nax = 0, nrb = 0;  // grids of the passes
+    WsLayout wl{};
+    double t0 = 0.0;       // start of the set-up
+    std::vector<double> done_at;
+    long long cyc = 0;
+    int status = CG_OK;
+    bool done = false;
+};
+
+// Grids of the passes and the layout of the bucket's one allocation.
+int layout_bucket(Bucket &b, const cg_opts &o, int N, int nb) {
+    const int prec = o.precision == CG_PREC_MIXED ? 1 : 0;
+    const int m = o.restart, L = b.ov.L;
+    const long long n = (long long)N * N;
+    const int sms_eff = std::max(1, b.ov.sms / nb);  // each system's share of the GPU
+    b.ndot2 = dots2_blocks(prec, sms_eff, m, n);
+    b.nax2 = axpy2_blocks(prec, sms_eff, m, n);
+    b.nax = std::max(1, (int)std::min<long long>((n + 255) / 256, 4LL * sms_eff));
+    const int rpc = rows_per_block(b.ov.var[0][2], L);
+    b.nrb = (N + rpc - 1) / rpc;
+    const size_t pld = (size_t)dots2_part_ld(m);
+    const size_t ngroups = ((size_t)b.ndot2 + 15) / 16;
+    b.wl = ws_layout(m, std::max(1, o.max_iter), std::max<size_t>(b.nrb, (size_t)b.nax) + 32,
+                                  4 * (size_t)b.ndot2 * pld, 4 * ngroups * pld, ngroups);
+    const size_t lq = (size_t)L / 2 + 1;
+    b.gq_elems = lq * lq;
+    BucketBufs &bb = b.bb;
+    struct { void **p; size_t bytes; } const a[] = {
+        {&bb.V, (prec ? sizeof(float2) : sizeof(double2)) * (size_t)(m + 2) * (size_t)n * nb},
+        {&bb.T, sizeof(double2) * (size_t)N * L * nb},
+        {&bb.WS, b.wl.bytes * nb},
+        {&bb.G, sizeof(double2) * b.gq_elems * nb},
+        {&bb.C, sizeof(double) * (size_t)n * nb},
+        {&bb.X, sizeof(double2) * (size_t)n * nb},
+        {&bb.B, sizeof(double2) * (size_t)n * nb},
+        {&bb.TW, sizeof(double2) * b.ov.ntw},
+        {&bb.G32, prec ? sizeof(float2) * b.gq_elems * nb : 0},
+        {&bb.C32, prec ? sizeof(float) * (size_t)n * nb : 0},
+        {&bb.TW32, prec ? sizeof(float2) * b.ov.ntw : 0},
+    };
+    size_t total = 0;
+    for (const auto &e : a) total += al256(e.bytes);
+    BK_CU(cudaMalloc(&bb.all, total));
+    char *at = (char *)bb.all;
+    for (const auto &e : a) {
+        *e.p = at;
+        at += al256(e.bytes);
+    }
+    return CG_OK;
+}
+
+int enqueue_states(Bucket &b);
+
+// Sets up the systems b.idx[0..B) (all of side N) as one bucket on ctx's device
+// and enqueues their first residual on the bucket's stream.
+int setup_bucket(cg_ctx *ctx, const cg_system *sys, const cg_opts &o, Bucket &b) {
+    const std::vector<int> &idx = b.idx;
+    BucketBufs &bb = b.bb;
     const int nb = (int)idx.size();
     const int N = sys[idx[0]].N;
     const long long n = (long long)N * N;
     const int prec = o.precision == CG_PREC_MIXED ? 1 : 0;  // Arnoldi cycles in complex64
     const size_t esz = prec ? sizeof(float2) : sizeof(double2);
-    const double t0 = now_s();
-    BucketBufs bb;
+    b.t0 = now_s();
     // operator of every system: the context builds it (GPU Green's block or the
     // given one, spectrum, tuned launch shapes), the bucket keeps a copy
     OpView ov{};
@@ -230,16 +294,12 @@ int solve_bucket(cg_ctx *ctx, const cg_system *sys, const std::vector<int> &idx,
         if (st != CG_OK) return st;
         BK_TRY(ctx_op_view(ctx, &ov));
         if (q == 0) {
-            const size_t lq = (size_t)ov.L / 2 + 1;
-            gq_elems = lq * lq;
-            BK_CU(cudaMalloc(&bb.G, sizeof(double2) * gq_elems * nb));
-            BK_CU(cudaMalloc(&bb.C, sizeof(double) * (size_t)n * nb));
-            BK_CU(cudaMalloc(&bb.X, sizeof(double2) * (size_t)n * nb));
-            BK_CU(cudaMalloc(&bb.B, sizeof(double2) * (size_t)n * nb));
-            if (prec) {
-                BK_CU(cudaMalloc(&bb.G32, sizeof(float2) * gq_elems * nb));
-                BK_CU(cudaMalloc(&bb.C32, sizeof(float) * (size_t)n * nb));
-            }
+            b.ov = ov;
+            BK_TRY(layout_bucket(b, o, N, nb));
+            gq_elems = b.gq_elems;
+            // (the context's own twiddles change with the next bucket's grid side)
+            BK_CU(cudaMemcpyAsync(bb.TW, ov.tw64, sizeof(double2) * ov.ntw, cudaMemcpyDeviceToDevice, ov.stream));
+            if (prec) BK_CU(cudaMemcpyAsync(bb.TW32, ov.tw32, sizeof(float2) * ov.ntw, cudaMemcpyDeviceToDevice, ov.stream));
         }
         if (prec) {
             BK_CU(cudaMemcpyAsync((float2 *)bb.G32 + gq_elems * q, ov.gq32, sizeof(float2) * gq_elems,
@@ -264,25 +324,15 @@ int solve_bucket(cg_ctx *ctx, const cg_system *sys, const std::vector<int> &idx,
         // the context's buffers are rebuilt by the next set-up: wait for the copies
         BK_CU(cudaStreamSynchronize(ov.stream));
     }
-    cudaStream_t s = ov.stream;
+    BK_CU(cudaStreamCreateWithFlags(&bb.run, cudaStreamNonBlocking));
+    cudaStream_t s = bb.run;
     const int L = ov.L;
     const int m = o.restart;
     const int sms_eff = std::max(1, ov.sms / nb);  // each system's share of the GPU
-    const int ndot2 = dots2_blocks(prec, sms_eff, m, n);
-    const int nax2 = axpy2_blocks(prec, sms_eff, m, n);
-    const int nax = std::max(1, (int)std::min<long long>((n + 255) / 256, 4LL * sms_eff));
-    const int rpc = rows_per_block(ov.var[0][2], L);
-    const int nrb = (N + rpc - 1) / rpc;
-    const size_t pld = (size_t)dots2_part_ld(m);
-    const size_t ngroups = ((size_t)ndot2 + 15) / 16;
-    const WsLayout wl = ws_layout(m, std::max(1, o.max_iter), std::max<size_t>(nrb, (size_t)nax) + 32,
-                                  4 * (size_t)ndot2 * pld, 4 * ngroups * pld, ngroups);
+    const int ndot2 = b.ndot2, nax2 = b.nax2, nax = b.nax, nrb = b.nrb;
+    const WsLayout &wl = b.wl;
     const size_t vsys = (size_t)(m + 2) * (size_t)n;
-    BK_CU(cudaMalloc(&bb.V, esz * vsys * nb));
-    BK_CU(cudaMalloc(&bb.T, sizeof(double2) * (size_t)N * L * nb));
-    BK_CU(cudaMalloc(&bb.WS, wl.bytes * nb));
     BK_CU(cudaMemsetAsync(bb.WS, 0, wl.bytes * nb, s));
-    BK_CU(cudaMallocHost((void **)&bb.st_host, sizeof(DevState) * nb));
     char *ws = (char *)bb.WS;
     KrylovPtrs kp{};
     kp.st = (DevState *)(ws + wl.st);
@@ -334,7 +384,7 @@ int solve_bucket(cg_ctx *ctx, const cg_system *sys, const std::vector<int> &idx,
     a64.vinv = ov.var[0][2];
     a64.gq = bb.G;
     a64.cdiag = bb.C;
-    a64.tw = ov.tw64;
+    a64.tw = bb.TW;
     a64.T = bb.T;
     a64.sms = ov.sms;
     a64.nsys = nb;
@@ -350,7 +400,7 @@ int solve_bucket(cg_ctx *ctx, const cg_system *sys, const std::vector<int> &idx,
         ap.vinv = ov.var[1][2];
         ap.gq = bb.G32;
         ap.cdiag = bb.C32;
-        ap.tw = ov.tw32;
+        ap.tw = bb.TW32;
     }
     VecSel vk;  // u_k of each system: V_s + k n
     vk.base = bb.V;
@@ -397,57 +447,62 @@ int solve_bucket(cg_ctx *ctx, const cg_system *sys, const std::vector<int> &idx,
     };
     // capture [steps while a system runs, update, next residual and decisions]
     // once; replay per cycle
-    BK_CU(cudaStreamCreateWithFlags(&bb.cap, cudaStreamNonBlocking));
-    BK_TRY(cycle_graph(kp, bb.cap, enqueue_steps, enqueue_update, &bb.gexec));
+    BK_TRY(cycle_graph(kp, s, enqueue_steps, enqueue_update, &bb.gexec));
     BK_CU(cudaEventCreateWithFlags(&bb.ev, cudaEventDisableTiming));
     BK_TRY(enqueue_begin(s));
-    std::vector<double> done_at(nb, -1.0);
-    int status = CG_OK;
+    b.done_at.assign(nb, -1.0);
+    return enqueue_states(b);
+}
+
+// Reads the states behind the last cycle of the bucket and records its event.
+int enqueue_states(Bucket &b) {
+    BK_CU(cudaMemcpy2DAsync(b.bb.st_host, sizeof(DevState), (const char *)b.bb.WS + b.wl.st, b.wl.bytes,
+                            sizeof(DevState), b.idx.size(), cudaMemcpyDeviceToHost, b.bb.run));
+    BK_CU(cudaEventRecord(b.bb.ev, b.bb.run));
+    return CG_OK;
+}
+
+// The event of the bucket has passed: launches its next cycle, or marks it done.
+int next_cycle(Bucket &b, const cg_opts &o) {
+    const double t = now_s();
+    int running = 0;
+    for (size_t q = 0; q < b.idx.size(); q++) {
+        if (b.bb.st_host[q].status != 0) {
+            if (b.done_at[q] < 0.0) b.done_at[q] = t;
+        } else {
+            running++;
+        }
+    }
     // every cycle of a running system takes at least one Arnoldi step, so the
     // budget bounds the cycles; the cap only guards against a state that never
     // reports an end
-    const long long max_cycles = (long long)o.max_iter + 2;
-    for (long long cyc = 0;; cyc++) {
-        if (cyc > max_cycles) {
-            status = CG_ERR_CUDA;
-            break;
-        }
-        BK_CU(cudaMemcpy2DAsync(bb.st_host, sizeof(DevState), ws + wl.st, wl.bytes, sizeof(DevState), nb,
-                                cudaMemcpyDeviceToHost, s));
-        BK_CU(cudaEventRecord(bb.ev, s));
-        BK_CU(cudaEventSynchronize(bb.ev));
-        const double t = now_s();
-        int running = 0;
-        for (int q = 0; q < nb; q++) {
-            if (bb.st_host[q].status != 0) {
-                if (done_at[q] < 0.0) done_at[q] = t;
-            } else {
-                running++;
-            }
-        }
-        if (running == 0) break;
-        if (o.timeout_s > 0.0 && t - t0 > o.timeout_s) {
-            status = CG_ERR_TIMEOUT;
-            break;
-        }
-        BK_CU(cudaGraphLaunch(bb.gexec, s));
-    }
-    // solutions and results
-    for (int q = 0; q < nb; q++) {
-        const cg_system &sy = sys[idx[q]];
-        BK_CU(cudaMemcpyAsync(sy.x, (const double2 *)bb.X + (size_t)n * q, sizeof(double2) * n, cudaMemcpyDefault, s));
-    }
-    BK_CU(cudaStreamSynchronize(s));
+    if (running == 0) b.done = true;
+    else if (o.timeout_s > 0.0 && t - b.t0 > o.timeout_s) b.status = CG_ERR_TIMEOUT, b.done = true;
+    else if (++b.cyc > (long long)o.max_iter + 2) b.status = CG_ERR_CUDA, b.done = true;
+    if (b.done) return CG_OK;
+    BK_CU(cudaGraphLaunch(b.bb.gexec, b.bb.run));
+    return enqueue_states(b);
+}
+
+// Solutions and results of a bucket that is done.
+int finish_bucket(const cg_system *sys, Bucket &b, cg_result *results) {
+    const int nb = (int)b.idx.size();
+    const int N = sys[b.idx[0]].N;
+    const long long n = (long long)N * N;
+    for (int q = 0; q < nb; q++)
+        BK_CU(cudaMemcpyAsync(sys[b.idx[q]].x, (const double2 *)b.bb.X + (size_t)n * q, sizeof(double2) * n,
+                              cudaMemcpyDefault, b.bb.run));
+    BK_CU(cudaStreamSynchronize(b.bb.run));
     const double t1 = now_s();
     for (int q = 0; q < nb; q++) {
-        const DevState &h = bb.st_host[q];
+        const DevState &h = b.bb.st_host[q];
         cg_result r = {};
         switch (h.status) {
             case 1: r.status = CG_OK; break;
             case 2: r.status = CG_ERR_NOT_CONVERGED; break;
             case 3: r.status = CG_ERR_BREAKDOWN; break;
             case 4: r.status = CG_ERR_NONFINITE; break;
-            default: r.status = status != CG_OK ? status : CG_ERR_CUDA; break;
+            default: r.status = b.status != CG_OK ? b.status : CG_ERR_CUDA; break;
         }
         r.iterations = h.it;
         r.cycles = h.cycles;
@@ -455,10 +510,46 @@ int solve_bucket(cg_ctx *ctx, const cg_system *sys, const std::vector<int> &idx,
         r.rel_residual_true = h.true_res;
         // latency: from the bucket's start (its set-up included) to the cycle
         // boundary at which the host saw the system finish
-        r.seconds = (done_at[q] > 0.0 ? done_at[q] : t1) - t0;
-        results[idx[q]] = r;
+        r.seconds = (b.done_at[q] > 0.0 ? b.done_at[q] : t1) - b.t0;
+        results[b.idx[q]] = r;
     }
-    (void)t_sweep;
+    return CG_OK;
+}
+
+// What a sweep holds until it returns.
+struct Sweep {
+    cg_ctx *ctx = nullptr;
+    DevState *states = nullptr;  // pinned, one per system
+    std::vector<std::unique_ptr<Bucket>> wave;
+    ~Sweep() {
+        wave.clear();
+        if (states) cudaFreeHost(states);
+        if (ctx) cugmres_destroy(ctx);
+    }
+};
+
+// Runs the buckets of a wave to their ends, each on its own stream.
+int run_wave(std::vector<std::unique_ptr<Bucket>> &wave, const cg_system *sys, const cg_opts &o, cg_result *results) {
+    size_t left = wave.size();
+    while (left > 0) {
+        for (auto &b : wave) {
+            if (b->done) continue;
+            if (left > 1) {
+                const cudaError_t e = cudaEventQuery(b->bb.ev);
+                if (e == cudaErrorNotReady) continue;
+                BK_CU(e);
+            } else {
+                BK_CU(cudaEventSynchronize(b->bb.ev));
+            }
+            BK_TRY(next_cycle(*b, o));
+            if (b->done) {
+                BK_TRY(finish_bucket(sys, *b, results));
+                left--;
+            }
+        }
+        if (left > 1) std::this_thread::yield();
+    }
+    wave.clear();
     return CG_OK;
 }
 
@@ -480,7 +571,6 @@ extern "C" int cugmres_solve_buckets(int device, int nsys, const cg_system *sys,
             (!sys[i].g_block && !(sys[i].k0 > 0.0 && sys[i].h > 0.0)))
             return CG_ERR_INVALID;
     if (nsys == 0) return CG_OK;
-    const double t_sweep = now_s();
     // group by grid side, hardest first inside a group
     std::map<int, std::vector<int>, std::greater<int>> groups;
     std::vector<double> hard(nsys, 0.0);
@@ -494,15 +584,26 @@ extern "C" int cugmres_solve_buckets(int device, int nsys, const cg_system *sys,
         const double kh = sys[i].k0 * sys[i].h > 0.0 ? sys[i].k0 * sys[i].h : 0.0;
         hard[i] = sys[i].N * kh * sqrt(1.0 + cmax);
     }
-    cg_ctx *ctx = nullptr;
-    int st = cugmres_create(&ctx, device);
-    if (st != CG_OK) return st;
+    Sweep sw;
+    BK_TRY(cugmres_create(&sw.ctx, device));
+    cg_ctx *ctx = sw.ctx;
+    BK_CU(cudaMallocHost((void **)&sw.states, sizeof(DevState) * nsys));
+    DevState *next_states = sw.states;
+    std::vector<std::unique_ptr<Bucket>> &wave = sw.wave;
     cg::ctx_set_shared_gpu(ctx, true);  // lockstep launches: no persistent column pass
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
         cudaGetLastError();
         free_b = (size_t)8 << 30;
     }
+    // Buckets run side by side in waves: a bucket of small grids leaves most of the
+    // GPU idle, and the steps of one fill it beside another's.  Ten systems of sides 96
+    // to 512, 200 steps: 118 ms one bucket after the other, 91 side by side, 55.5 with
+    // the set-up's allocations merged as well (its share, one step a system: 60 -> 21).
+    // A wave's buckets share half of the free memory; with a time limit, which counts
+    // from a bucket's set-up, each runs alone.
+    constexpr size_t WAVE_BUCKETS = 8;
+    size_t wave_bytes = 0;
     for (auto &kv : groups) {
         std::vector<int> &ids = kv.second;
         std::stable_sort(ids.begin(), ids.end(), [&](int a, int b) { return hard[a] > hard[b]; });
@@ -519,13 +620,33 @@ extern "C" int cugmres_solve_buckets(int device, int nsys, const cg_system *sys,
         if (max_bucket > 0) cap = std::min(cap, max_bucket);
         for (size_t b0 = 0; b0 < ids.size(); b0 += cap) {
             std::vector<int> bucket(ids.begin() + b0, ids.begin() + std::min(ids.size(), b0 + (size_t)cap));
-            st = solve_bucket(ctx, sys, bucket, o, t_sweep, results);
-            if (st != CG_OK) {
-                cugmres_destroy(ctx);
+            const size_t bytes = bucket.size() * (per + 2 * sizeof(double2) * (size_t)(o.restart + 1) * (o.restart + 1));
+            if (!wave.empty() && (o.timeout_s > 0.0 || wave.size() == WAVE_BUCKETS || wave_bytes + bytes > free_b / 2))
+                BK_TRY(run_wave(wave, sys, o, results));
+            if (wave.empty()) wave_bytes = 0;
+            auto b = std::make_unique<Bucket>();
+            b->idx = bucket;
+            b->bb.st_host = next_states;
+            next_states += bucket.size();
+            int st = setup_bucket(ctx, sys, o, *b);
+            if (st == CG_ERR_OOM && !wave.empty()) {  // the wave's buffers stand in its way: alone
+                cudaGetLastError();
+                BK_TRY(run_wave(wave, sys, o, results));
+                wave_bytes = 0;
+                DevState *const states = b->bb.st_host;
+                b = std::make_unique<Bucket>();
+                b->idx = bucket;
+                b->bb.st_host = states;
+                st = setup_bucket(ctx, sys, o, *b);
+            }
+            if (st != CG_OK) {  // the buckets before it have their results all the same
+                b.reset();
+                if (!wave.empty()) BK_TRY(run_wave(wave, sys, o, results));
                 return st;
             }
+            wave.push_back(std::move(b));
+            wave_bytes += bytes;
         }
     }
-    cugmres_destroy(ctx);
-    return CG_OK;
+    return wave.empty() ? CG_OK : run_wave(wave, sys, o, results);
 }

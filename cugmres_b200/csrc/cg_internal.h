@@ -177,6 +177,7 @@ struct OpView {
     const float *c32;
     const double2 *tw64;
     const float2 *tw32;
+    size_t ntw;  // entries of each twiddle table
     cudaStream_t stream;
 };
 int ctx_op_view(const cg_ctx *c, OpView *v);
