@@ -1405,13 +1405,6 @@ int prepare_grid(cg_fno *f, int B, int H, int W) {
     return CG_OK;
 }
 
-int set_smem_attrs(int H) {
-    if (cudaFuncSetAttribute(k_dft_h_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, H * 8) ||
-        cudaFuncSetAttribute(k_dft_h_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, H * 8))
-        return -1;
-    return 0;
-}
-
 // Spectral branch S_l(in) into f->spec (FP32 [cells][C]); saves X2 when X2save.
 // tc: the column DFT runs on the tensor cores from f->vT, the channel-major copy of `in`.
 int spectral_fwd(cg_fno *f, const __nv_bfloat16 *in, int B, int H, int W, int layer, float2 *X2save, const int *gate,
@@ -1454,7 +1447,6 @@ template <typename RT>
 int forward(cg_fno *f, cudaStream_t s, int B, int H, int W, const RT *r, const float *chi, RT *zout, bool train,
             const cg_c64 *x, const int *gate) {
     const long long hw = (long long)H * W, cells = B * hw;
-    if (set_smem_attrs(H)) return CG_ERR_CUDA;
     const int nbx = (int)std::max<long long>(1, std::min<long long>(NBX_MAX, (hw + 1023) / 1024));
     k_norm_part<RT><<<dim3(nbx, B), RED_THREADS, 0, s>>>(r, train ? x : nullptr, hw, nbx, f->npart, gate);
     k_norm_fin<<<(B + 63) / 64, 64, 0, s>>>(f->npart, nbx, B, hw, f->s, f->inv_s, train ? f->wts : nullptr, gate);

@@ -17,12 +17,19 @@ namespace cg {
 // opting in.  Comparing `dyn` alone let kernels with static arrays fail to
 // launch just below the threshold (the delayed-CGS2 step kernel, 6.4 KB
 // static, at restarts of about 1070 to 1230).
+// The limit belongs to the kernel and the device, not to a context, so it is
+// always set to all that a block can have: set to `dyn`, the limit of one
+// host thread's launch could fall below another's between its opt-in and its
+// launch (contexts with different restarts: CG_ERR_CUDA from a valid solve).
+constexpr size_t SMEM_BLOCK_MAX = 227 * 1024;  // static and dynamic, sm_100
 template <typename K> inline int smem_optin(K kern, size_t dyn) {
     cudaFuncAttributes a;
     cudaError_t e = cudaFuncGetAttributes(&a, kern);
     if (e != cudaSuccess) return (int)e;
     if (a.sharedSizeBytes + dyn <= 48 * 1024) return 0;
-    return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+    if (a.sharedSizeBytes + dyn > SMEM_BLOCK_MAX) return (int)cudaErrorInvalidValue;
+    return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)(SMEM_BLOCK_MAX - a.sharedSizeBytes));
 }
 
 // Solver state kept in device memory so that no host synchronisation is

@@ -508,9 +508,8 @@ cudaLaunchConfig_t cluster_config(int nsys, int bytes, cudaLaunchAttribute *at, 
     return cfg;
 }
 template <typename K> int cluster_optin(K kern, int bytes) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    return (int)e;
+    if (int e = smem_optin(kern, bytes)) return e;
+    return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
 }
 
 template <typename C, int NP>
