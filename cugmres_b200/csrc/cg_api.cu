@@ -484,8 +484,13 @@ int autotune(cg_ctx *c, int prec) {
     }
     // the key carries the tuner's version so that choices made by an older
     // tuner or for older kernels are not reused
+    // The persistent column pass is a choice only of a context that has the GPU to
+    // itself and more columns than SMs (with fewer no block has a second column to
+    // load ahead), so up to there contexts with and without company share a choice:
+    // a small system comes out bit for bit the same in a sweep and alone.
+    const bool one_wave = c->L <= c->sms, persistent = !c->shared_gpu && !one_wave;
     std::string key = std::string(c->devname) + "|" + std::to_string(c->L) + "|" + std::to_string(prec) + "|t4" +
-                      (c->shared_gpu ? "s" : "");
+                      (one_wave ? "c" : c->shared_gpu ? "s" : "");
     for (char &ch : key)
         if (ch == ' ') ch = '_';
     {
@@ -547,7 +552,7 @@ int autotune(cg_ctx *c, int prec) {
         bool changed = false;
         for (int pass = 0; pass < 3 && status == CG_OK; pass++)
             for (int v = 0; v < nv && status == CG_OK; v++) {
-                if (v == best[pass] || (c->shared_gpu && matvec_variant_persistent(v))) continue;
+                if (v == best[pass] || (!persistent && matvec_variant_persistent(v))) continue;
                 std::array<int, 3> cand = best;
                 cand[pass] = v;
                 const float ms = time_shapes(cand);
