@@ -852,15 +852,20 @@ k_proj_bwd(const __nv_bfloat16 *__restrict__ zq, const float *__restrict__ dout,
 
 // Weight gradient of a channel mixing: dWt[o][i] = sum_cells dY[o] X[i],
 // db[o] = sum_cells dY[o]; per-block partials [NO*NI + NO].  A contraction over
-// the cells of two BF16 arrays, so it runs on the tensor cores (mma.sync m16n8k16,
-// FP32 accumulators; the operands are cell-major, which ldmatrix.trans turns into
-// fragments).  mma.sync and not tcgen05: the outputs are one 32- or 128-row tile
-// that a warp's registers hold, and the kernel is bound by reading the cells
-// once.  Tiles of 64 cells, double-buffered with cp.async.  NO = 128: warp w owns
-// rows 32 w ..; NO = 32: warp w takes every fourth group of 16 cells and the block
-// adds the warps' tiles in order.  db is one more column tile against ones.
-// 16 x 64 x 64 cells: 74 -> 8 us (NO = 128) and 45 -> 6 us (NO = 32) against FP32
-// fused multiply-adds from shared memory.
+// the cells of two BF16 arrays, so it runs on the tensor cores (mma.sync; the
+// operands are cell-major, which ldmatrix.trans turns into fragments).  mma.sync
+// and not tcgen05: the outputs are one 32- or 128-row tile that a warp's registers
+// hold, and the kernel is bound by reading the cells once.  Tiles of 64 cells,
+// double-buffered with cp.async.  NO = 128: warp w owns rows 32 w ..; NO = 32: warp w
+// takes every fourth group of 16 cells and the block adds the warps' tiles in
+// order.  db is one more column tile against ones.
+// The tensor cores cut the sum of an accumulator and their products off instead of
+// rounding it, which a chain of them adds up, so eight cells at a time (m16n8k8) are
+// added to the sums by FP32 additions.  Error of dW against 64 bits, random values of
+// mean 1, relative rms, 16 x 64 x 64 / 16 x 160 x 160 cells, NO = 128: FP32 fused multiply-adds 2.8e-8 /
+// 3.5e-8, a chain of m16n8k16 2.5e-7 / 1.6e-6, this 2.7e-8 / 2.4e-8 (steps of 16 cells 3.0e-8 / 2.7e-8).
+// Time on 16 x 64 x 64 cells, launch included: 49 us (NO = 128) and 31 us (NO = 32) by FP32 fused
+// multiply-adds from shared memory, 10 and 9 by the chain, 13 and 10.5 by this.
 constexpr int WG_CELLS = 64, WG_THREADS = 128;
 __device__ __forceinline__ uint32_t wg_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void wg_copy16(void *dst, const void *src, bool ok) {
@@ -872,11 +877,20 @@ __device__ __forceinline__ void wg_ldsm_t(uint32_t (&r)[4], const __nv_bfloat16 
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                  : "r"(wg_smem(row)));
 }
+// c += A B for 16 cells as two products of eight, each from a zero accumulator and
+// added by FP32 additions (see above).
 __device__ __forceinline__ void wg_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-                 "{%0, %1, %2, %3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+    auto mma8 = [](float (&d)[4], uint32_t a0, uint32_t a1, uint32_t b) {
+        asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, "
+                     "{%7, %7, %7, %7};"
+                     : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+                     : "r"(a0), "r"(a1), "r"(b), "f"(0.f));
+    };
+    float d[4], e[4];
+    mma8(d, a[0], a[1], b0);
+    mma8(e, a[2], a[3], b1);
+#pragma unroll
+    for (int q = 0; q < 4; q++) c[q] += d[q] + e[q];
 }
 template <int NO>
 __global__ void __launch_bounds__(WG_THREADS)
