@@ -1312,10 +1312,10 @@ int cugmres_solve(cg_ctx *c, const cg_c128 *b, cg_c128 *x, const cg_opts *opts_i
     bool use_prec = learned;  // this cycle runs the learned preconditioner
     // small grids: the steps up to the device's stop as one kernel (profiled cycles
     // keep their phases, flexible GMRES ends some cycles after a number of launches)
-    const bool small = want_delayed && !learned && !c->prof && small_cycle_fits(prec, c->N, c->L, c->mcap);
+    const bool small = want_delayed && !learned && !c->prof && small_cycle_fits(prec, c->N, c->L, m);
     auto enqueue_steps = [&](int steps, cudaStream_t q) -> int {
         if (small) {
-            CG_LAUNCH(launch_small_cycle(prec, c->V, n, kp, ap, q));
+            CG_LAUNCH(launch_small_cycle(prec, c->V, n, kp, m, ap, q));
             return CG_OK;
         }
         for (int i = 0; i < steps; i++) {

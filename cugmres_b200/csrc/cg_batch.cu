@@ -427,7 +427,7 @@ int setup_bucket(cg_ctx *ctx, const cg_system *sys, const cg_opts &o, Bucket &b)
     const bool small = small_cycle_fits(prec, N, L, m);  // a cluster per system runs its whole cycle
     auto enqueue_steps = [&](cudaStream_t q) -> int {
         if (small) {
-            BK_LAUNCH(launch_small_cycle(prec, bb.V, n, kp, ap, q));
+            BK_LAUNCH(launch_small_cycle(prec, bb.V, n, kp, m, ap, q));
             return CG_OK;
         }
         for (int i = 0; i < LOOP_STEPS; i++) {

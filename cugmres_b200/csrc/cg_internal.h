@@ -215,11 +215,12 @@ int launch_loop_test(const KrylovPtrs &kp, cudaGraphConditionalHandle h, cudaStr
 // ortho 0: delayed CGS2, 1: CGS2, for the cycle k_cycle_begin has just set up
 int launch_set_ortho(const KrylovPtrs &kp, int ortho, cudaStream_t s);
 // Whole delayed-CGS2 cycles of small grids in one kernel (cg_small.cu): 1 where
-// it serves grid side N (embedding L) with room for `mcap` basis vectors; the
-// launch runs the cycle that k_cycle_begin has set up to its stop.
-int small_cycle_fits(int prec, int N, int L, int mcap);
+// it serves grid side N (embedding L) and cycles of up to `m` steps, which size its
+// shared memory (a context's room for basis vectors, kp.mcap, may come from a longer
+// solve before); the launch runs the cycle that k_cycle_begin has set up to its stop.
+int small_cycle_fits(int prec, int N, int L, int m);
 int launch_small_matvec(int prec, const void *x, void *y, const MatvecArgs &a, cudaStream_t s);  // y = A x, same grids
-int launch_small_cycle(int prec, void *V, long long n, const KrylovPtrs &kp, const MatvecArgs &a, cudaStream_t s);
+int launch_small_cycle(int prec, void *V, long long n, const KrylovPtrs &kp, int m, const MatvecArgs &a, cudaStream_t s);
 // s-step Arnoldi (cg_sstep.cu): S steps per block, S in {2, 4, 8}
 constexpr int SS_MAX = 8;
 // An FP64 block whose first pass keeps more than this fraction of every

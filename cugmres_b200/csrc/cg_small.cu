@@ -46,7 +46,7 @@ constexpr int SC_CTAS = 16, SC_THREADS = 256, SC_WARPS = SC_THREADS / 32;
 struct SmallSmem {
     int su, sw, sc, tb, rb, ex, part, d1, d2, tv, cs, sn, col, pc, bytes;
 };
-template <typename C, int NP> __host__ __device__ constexpr SmallSmem small_smem(int N, int mcap) {
+template <typename C, int NP> __host__ __device__ constexpr SmallSmem small_smem(int N, int m) {
     typedef WPlan<NP> P;
     const int rpc = (N + SC_CTAS - 1) / SC_CTAS, ns = rpc * N, e = sizeof(C);
     SmallSmem s{};
@@ -62,14 +62,14 @@ template <typename C, int NP> __host__ __device__ constexpr SmallSmem small_smem
     s.tb = take(2 * NP / SC_CTAS * (N + 1) * e);
     s.rb = take(rpc * (2 * NP + 1) * e);
     s.ex = take(SC_WARPS * P::WREG * e);
-    s.part = take(4 * (mcap + 2) * 8);
-    s.d1 = take((mcap + 2) * 16);
-    s.d2 = take((mcap + 2) * 16);
-    s.tv = take(2 * (mcap + 2) * 16);
-    s.cs = take((mcap + 1) * 16);
-    s.sn = take((mcap + 1) * 8);
-    s.col = take((mcap + 2) * 16);
-    s.pc = take(2 * (mcap + 2) * e);  // P and S of the axpy
+    s.part = take(4 * (m + 2) * 8);
+    s.d1 = take((m + 2) * 16);
+    s.d2 = take((m + 2) * 16);
+    s.tv = take(2 * (m + 2) * 16);
+    s.cs = take((m + 1) * 16);
+    s.sn = take((m + 1) * 8);
+    s.col = take((m + 2) * 16);
+    s.pc = take(2 * (m + 2) * e);  // P and S of the axpy
     s.bytes = o;
     return s;
 }
@@ -219,7 +219,7 @@ template <typename C, int NP> struct SmallOp {
 template <typename C, int NP>
 __global__ void __launch_bounds__(SC_THREADS, 1)
 k_small_cycle(C *V, long long n, KrylovPtrs kp, int N, const typename real_of<C>::type *cdiag, const C *gq,
-              const C *__restrict__ tw, int transpose, long long sys_c, long long sys_gq) {
+              const C *__restrict__ tw, int transpose, int m, long long sys_c, long long sys_gq) {
     typedef typename real_of<C>::type R;
     kp = kp_sys(kp);
     V = sys_vec(V, kp);
@@ -230,13 +230,13 @@ k_small_cycle(C *V, long long n, KrylovPtrs kp, int N, const typename real_of<C>
     cgr::cluster_group cl = cgr::this_cluster();
     const int rank = (int)cl.block_rank();
     extern __shared__ __align__(16) unsigned char smem[];
-    const SmallSmem lay = small_smem<C, NP>(N, kp.mcap);
+    const SmallSmem lay = small_smem<C, NP>(N, m);
     double *part = reinterpret_cast<double *>(smem + lay.part);
     double2 *D1 = reinterpret_cast<double2 *>(smem + lay.d1), *D2 = reinterpret_cast<double2 *>(smem + lay.d2);
     double2 *tvs = reinterpret_cast<double2 *>(smem + lay.tv), *css = reinterpret_cast<double2 *>(smem + lay.cs);
     double *sns = reinterpret_cast<double *>(smem + lay.sn);
     double2 *col = reinterpret_cast<double2 *>(smem + lay.col);
-    C *Pc = reinterpret_cast<C *>(smem + lay.pc), *Sc = Pc + (kp.mcap + 2);
+    C *Pc = reinterpret_cast<C *>(smem + lay.pc), *Sc = Pc + (m + 2);
     __shared__ double red[SC_WARPS][4];
     __shared__ double scan_a[SC_THREADS];
     __shared__ double2 scan_b[SC_THREADS];
@@ -253,7 +253,7 @@ k_small_cycle(C *V, long long n, KrylovPtrs kp, int N, const typename real_of<C>
         su[e] = V[base + e];
         op.sc[e] = cdiag[base + e];
     }
-    const int m_max = st->m, maxit = st->maxit, ref = st->rotation == 1, fixed = st->fixed, ld = kp.mcap + 1;
+    const int m_max = st->m < m ? st->m : m, maxit = st->maxit, ref = st->rotation == 1, fixed = st->fixed, ld = kp.mcap + 1;
     const double tol_abs = st->tol * st->nb, inner_abs = st->inner_tol * st->beta0, nb = st->nb;
     int it = st->it;
     __syncthreads();
@@ -306,7 +306,7 @@ k_small_cycle(C *V, long long n, KrylovPtrs kp, int N, const typename real_of<C>
         }
         __syncthreads();
         // ------------------------------------------------ the step, as in dcgs2_step (every CTA the same)
-        const double2 *tv = tvs + (k & 1) * (kp.mcap + 2);
+        const double2 *tv = tvs + (k & 1) * (m + 2);
         double sa = 0.0, acr = 0.0, aci = 0.0, hn = 0.0;
         for (int j = tid; j < k; j += SC_THREADS) {
             const double2 a = D1[j], c = D2[j];
@@ -461,7 +461,7 @@ k_small_cycle(C *V, long long n, KrylovPtrs kp, int N, const typename real_of<C>
         }
         // t_k = ([c; delta] - H(0:k, 0:k-1) a) / nu, a warp per row, rows dealt to the CTAs, to every CTA's next buffer
         // (column k-1 of H is the one in col; the earlier ones were written before the last barriers)
-        double2 *tn = tvs + ((k + 1) & 1) * (kp.mcap + 2);
+        double2 *tn = tvs + ((k + 1) & 1) * (m + 2);
         for (int i = rank + SC_CTAS * warp; i <= k; i += SC_CTAS * SC_WARPS) {
             double er = 0.0, ei = 0.0;
             for (int j = (i > 0 ? i - 1 : 0) + lane; j < k; j += 32) {
@@ -519,15 +519,15 @@ template <typename K> int cluster_optin(K kern, int bytes) {
 }
 
 template <typename C, int NP>
-int launch(void *V, long long n, const KrylovPtrs &kp, const MatvecArgs &a, cudaStream_t s) {
+int launch(void *V, long long n, const KrylovPtrs &kp, int m, const MatvecArgs &a, cudaStream_t s) {
     typedef typename real_of<C>::type R;
     auto kern = k_small_cycle<C, NP>;
-    const int bytes = small_smem<C, NP>(a.N, kp.mcap).bytes;
+    const int bytes = small_smem<C, NP>(a.N, m).bytes;
     if (int e = cluster_optin(kern, bytes)) return e;
     cudaLaunchAttribute at;
     const cudaLaunchConfig_t cfg = cluster_config(kp.nsys, bytes, &at, s);
     return (int)cudaLaunchKernelEx(&cfg, kern, (C *)V, n, kp, a.N, (const R *)a.cdiag, (const C *)a.gq,
-                                   (const C *)a.tw, a.transpose, a.sys_c, a.sys_gq);
+                                   (const C *)a.tw, a.transpose, m, a.sys_c, a.sys_gq);
 }
 template <typename C, int NP> int launch_mv(const void *x, void *y, const MatvecArgs &a, cudaStream_t s) {
     typedef typename real_of<C>::type R;
@@ -542,7 +542,7 @@ template <typename C, int NP> int launch_mv(const void *x, void *y, const Matvec
 
 // 220 KB: a CTA's shared memory (227 KB) less this kernel's static arrays
 constexpr int SC_SMEM = 220 * 1024;
-template <typename C, int NP> bool fits(int N, int mcap) {
+template <typename C, int NP> bool fits(int N, int m) {
     static const int most = [] {  // clusters that the device holds at that size
         auto kern = k_small_cycle<C, NP>;
         cudaLaunchAttribute at;
@@ -554,12 +554,12 @@ template <typename C, int NP> bool fits(int N, int mcap) {
         }
         return c;
     }();
-    return most > 0 && small_smem<C, NP>(N, mcap).bytes <= SC_SMEM;
+    return most > 0 && small_smem<C, NP>(N, m).bytes <= SC_SMEM;
 }
 
 }  // namespace
 
-int small_cycle_fits(int prec, int N, int L, int mcap) {
+int small_cycle_fits(int prec, int N, int L, int m) {
     // CUGMRES_SMALL_CYCLE=0, or a forced shape of the launched passes: diagnostics
     static const bool on = [] {
         const char *e = getenv("CUGMRES_SMALL_CYCLE");
@@ -571,12 +571,12 @@ int small_cycle_fits(int prec, int N, int L, int mcap) {
         return true;
     }();
     if (!on || L != 128) return 0;
-    return prec == 0 ? fits<double2, 64>(N, mcap) : fits<float2, 64>(N, mcap);
+    return prec == 0 ? fits<double2, 64>(N, m) : fits<float2, 64>(N, m);
 }
 
-int launch_small_cycle(int prec, void *V, long long n, const KrylovPtrs &kp, const MatvecArgs &a, cudaStream_t s) {
-    if (a.L != 128) return (int)cudaErrorInvalidValue;
-    return prec == 0 ? launch<double2, 64>(V, n, kp, a, s) : launch<float2, 64>(V, n, kp, a, s);
+int launch_small_cycle(int prec, void *V, long long n, const KrylovPtrs &kp, int m, const MatvecArgs &a, cudaStream_t s) {
+    if (a.L != 128 || m > kp.mcap) return (int)cudaErrorInvalidValue;
+    return prec == 0 ? launch<double2, 64>(V, n, kp, m, a, s) : launch<float2, 64>(V, n, kp, m, a, s);
 }
 
 int launch_small_matvec(int prec, const void *x, void *y, const MatvecArgs &a, cudaStream_t s) {

@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 from conftest import ROOT
+from cugmres_b200 import problems
 
 pytestmark = pytest.mark.gpu
 
@@ -45,3 +46,52 @@ def test_long_cycles_lose_no_more(tmp_path, cuda_device, precision):
     1.13; sums over all basis vectors in a single chain are 1.5 times off in complex64."""
     one, launched = _both(FLOORS, tmp_path, precision)
     assert np.exp(np.mean(np.log(one / launched))) <= 1.25
+
+
+@pytest.mark.parametrize("N", [33, 64])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_long_solve_before_changes_nothing(solver, N, precision):
+    """A context's solves do not depend on the restart lengths it has seen."""
+    pr = problems.helmholtz(N, 3.0, seed=N)
+    solver.set_operator(pr["g_block"], pr["chi"], pr["chi_scale"])
+    kw = dict(max_iter=90, tol=1e-13, precision=precision)
+    before, _ = solver.solve(pr["b"], restart=30, **kw)
+    solver.solve(pr["b"], restart=1500, **kw)
+    after, _ = solver.solve(pr["b"], restart=30, **kw)
+    assert np.array_equal(before, after)
+
+
+HISTORIES = r"""
+import sys, numpy as np
+sys.path.insert(0, sys.argv[1])
+import cugmres_b200 as cg
+from cugmres_b200 import problems as P
+pr = P.helmholtz(64, 14.0, seed=1, cells_per_wavelength=12.0)
+with cg.Solver(0) as s:
+    s.set_operator(pr["g_block"], pr["chi"], pr["chi_scale"])
+    _, info = s.solve(pr["b"], restart=600, max_iter=600, tol=0.0, precision=sys.argv[3], inner_tol=0.0)
+np.save(sys.argv[2], info["res_hist"])
+"""
+
+
+@pytest.mark.parametrize("precision,rel", [("fp64", 1e-2), ("mixed", 1e-1)])
+def test_histories_of_600_steps(tmp_path, cuda_device, precision, rel):
+    """One cycle of 600 steps (several rotations a thread from step 258 on).  The residual
+    norms of GMRES move little under rounding: 5e-4 in FP64 and 1e-2 in complex64 over
+    such a cycle, where steps change them by a factor of 1e3 in all."""
+    one, launched = _both(HISTORIES, tmp_path, precision)
+    assert one.shape == launched.shape == (601,)
+    assert np.all(np.abs(one - launched) <= rel * launched)
+
+
+@pytest.mark.parametrize("N", [33, 64])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("restart", [900, 940, 980, 1060, 1180, 1260, 1340])
+def test_restarts_around_the_capacity(solver, N, precision, restart):
+    """Restart lengths on both sides of what a block's shared memory holds."""
+    pr = problems.helmholtz(N, 6.0, seed=N)
+    solver.set_operator(pr["g_block"], pr["chi"], pr["chi_scale"])
+    x, info = solver.solve(pr["b"], restart=restart, max_iter=2 * restart, tol=1e-10, precision=precision)
+    assert info["status"] == 0 and info["rel_residual_true"] <= 1e-10
+    r, rel = solver.residual(pr["b"], x)
+    assert rel <= 1.01e-10
