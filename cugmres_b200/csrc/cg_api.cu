@@ -1387,7 +1387,7 @@ int cugmres_solve(cg_ctx *c, const cg_c128 *b, cg_c128 *x, const cg_opts *opts_i
     // again from the probe's shifts.
     constexpr int SS_REFRESH_MIN = 256, SS_REFRESH_STEPS = 100, SS_REFRESH_WINDOW = 32;
     const bool ss_segments = m > SS_REFRESH_MIN;
-    kp.ss_tau = ss_segments ? SS_ONE_PASS_LONG : SS_ONE_PASS;
+    kp.ss_tau = sstep_one_pass(S, m);
     const int ss_nblk = S > 0 ? (m + S - 1) / S : 0;  // blocks of a full s-step cycle
     double2 shifts0[SS_MAX];
     for (int i = 0; i < SS_MAX; i++) shifts0[i] = make_double2(0.0, 0.0);

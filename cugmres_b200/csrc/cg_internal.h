@@ -86,7 +86,7 @@ struct KrylovPtrs {
     double *gpart;   // [ceil(nblk_dots2 / 16) * 4 * part_ld] group sums of the dot partials
     unsigned int *tickets;  // [ceil(nblk_dots2 / 16)] arrival counters of those groups (reset by the last)
     double2 *ss = nullptr;  // s-step scratch (cg_sstep.cu: block coefficients, Gram, shifts, work rows)
-    double ss_tau = 0.0;    // s-step, FP64: threshold of the one-pass blocks (SS_ONE_PASS)
+    double ss_tau = 0.0;    // s-step, FP64: threshold of the one-pass blocks (sstep_one_pass)
     int mcap;        // allocated restart capacity (leading dimension of Rm / part)
     // Bucket of systems solved in lockstep (one launch covers all of them,
     // system = blockIdx.y): every array above (st included) of system s lies
@@ -230,13 +230,20 @@ constexpr int SS_MAX = 8;
 // (699, 699, 673 with S = 2, 4, 8), which a 1e-2 threshold did not (711 with S = 2).
 // Complex64 blocks always take both passes (eps = 6e-8).
 constexpr double SS_ONE_PASS = 0.1;
-// ... and this in a long (segmented) cycle, where the loss of the first blocks
-// grows over thousands of steps until a later block's Cholesky fails and the
-// restart throws the Krylov space away.  512^2, eps_r = 4, restart 4500, to
-// 1e-10 with five sets of FFT launch shapes, which differ in rounding only: at
-// 0.1 7457, 7779, 6953, 5379 and 9000 steps (the last without converging), 7.5 to
-// 9.5 s; at 0.5 5404, 5449, 5519, 5651 and 5558, 7.5 to 7.9 s.
+// ... and this in a long cycle, where the loss of the first blocks grows over the
+// steps until a later block's Cholesky fails and the restart throws the Krylov space
+// away.  512^2, eps_r = 4, restart 4500, to 1e-10 with five sets of FFT launch shapes,
+// which differ in rounding only: at 0.1 7457, 7779, 6953, 5379 and 9000 steps (the last
+// without converging), 7.5 to 9.5 s; at 0.5 5404, 5449, 5519, 5651 and 5558, 7.5 to 7.9 s.
+// Long is above 512 steps, and above 256 with S = 2.  With S = 4 the loss first shows at
+// restart 2000 (512^2: 5 cycles at 0.1 where 0.5 takes 4; 3000: no convergence within 9000
+// steps, 8571 at 0.5), and the skipped passes save most in short cycles, s at 0.1 / 0.5
+// with the same steps and residual: 1024^2 restart 300 0.405 / 0.503 (900 steps), 400 0.49 /
+// 0.69 (800), 500 0.80 / 0.87 (1000), 1000 1.60 / 1.63 (1000); 2048^2 restart 300 0.42 /
+// 0.66 (300).  With S = 2 0.1 breaks cycles off from 300 steps on (512^2, 1200 steps:
+// 7 cycles against 4, residual 7.456e-3 against 7.442e-3; restart 400 7.32e-3 against 6.65e-3).
 constexpr double SS_ONE_PASS_LONG = 0.5;
+inline double sstep_one_pass(int S, int m) { return m > (S >= 4 ? 512 : 256) ? SS_ONE_PASS_LONG : SS_ONE_PASS; }
 int sstep_supported(int S);
 long long sstep_scratch_elems(int mcap);  // double2 entries of KrylovPtrs::ss
 int sstep_part_ld(int mcap);              // partials per block of the block dot pass
