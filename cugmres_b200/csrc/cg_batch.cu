@@ -29,6 +29,7 @@
 #include "../../include/cugmres.h"
 #include "cg_common.cuh"
 #include "cg_internal.h"
+#include "cg_wave.h"
 
 namespace {
 
@@ -280,7 +281,6 @@ int setup_bucket(cg_ctx *ctx, const cg_system *sys, const cg_opts &o, Bucket &b)
     const int N = sys[idx[0]].N;
     const long long n = (long long)N * N;
     const int prec = o.precision == CG_PREC_MIXED ? 1 : 0;  // Arnoldi cycles in complex64
-    const size_t esz = prec ? sizeof(float2) : sizeof(double2);
     b.t0 = now_s();
     // operator of every system: the context builds it (GPU Green's block or the
     // given one, spectrum, tuned launch shapes), the bucket keeps a copy
@@ -530,27 +530,25 @@ struct Sweep {
 
 // Runs the buckets of a wave to their ends, each on its own stream.
 int run_wave(std::vector<std::unique_ptr<Bucket>> &wave, const cg_system *sys, const cg_opts &o, cg_result *results) {
-    size_t left = wave.size();
-    while (left > 0) {
-        for (auto &b : wave) {
-            if (b->done) continue;
-            if (left > 1) {
-                const cudaError_t e = cudaEventQuery(b->bb.ev);
-                if (e == cudaErrorNotReady) continue;
-                BK_CU(e);
-            } else {
-                BK_CU(cudaEventSynchronize(b->bb.ev));
+    const int st = run_side_by_side(
+        wave,
+        [](Bucket &b, bool last, bool *go) -> int {
+            if (last) {
+                BK_CU(cudaEventSynchronize(b.bb.ev));
+                return CG_OK;
             }
-            BK_TRY(next_cycle(*b, o));
-            if (b->done) {
-                BK_TRY(finish_bucket(sys, *b, results));
-                left--;
+            const cudaError_t e = cudaEventQuery(b.bb.ev);
+            *go = e != cudaErrorNotReady;
+            if (!*go) {
+                cudaGetLastError();  // not an error of the launches that follow
+                return CG_OK;
             }
-        }
-        if (left > 1) std::this_thread::yield();
-    }
+            BK_CU(e);
+            return CG_OK;
+        },
+        [&](Bucket &b) { return next_cycle(b, o); }, [&](Bucket &b) { return finish_bucket(sys, b, results); });
     wave.clear();
-    return CG_OK;
+    return st;
 }
 
 }  // namespace
