@@ -424,8 +424,8 @@ def sweep_side(args, rank, world, device, precision="mixed"):
                   "precision": precision,
                   "note": (f"GMRES({args.sweep_restart}), tol {args.tol:g}, at most {args.sweep_max_iter} steps per "
                            "system; "
-                           "latency = from the start of the system's bucket (set-up included) to the cycle "
-                           "at which it finished")})
+                           "latency = set-up of the system's bucket, and from the wave's first cycle to the one "
+                           "at which it finished (the buckets of a wave share the GPU)")})
     return stats
 
 

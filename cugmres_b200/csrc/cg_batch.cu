@@ -221,7 +221,8 @@ struct Bucket {
     size_t gq_elems = 0;
     int ndot2 = 0, nax2 = 0, nax = 0, nrb = 0;  // grids of the passes
     WsLayout wl{};
-    double t0 = 0.0;       // start of the set-up
+    double t0 = 0.0;       // start of the set-up; from run_wave on, moved past what the bucket waited for the others'
+    double t_set_up = 0.0; // its end
     std::vector<double> done_at;
     long long cyc = 0;
     int status = CG_OK;
@@ -451,7 +452,9 @@ int setup_bucket(cg_ctx *ctx, const cg_system *sys, const cg_opts &o, Bucket &b)
     BK_CU(cudaEventCreateWithFlags(&bb.ev, cudaEventDisableTiming));
     BK_TRY(enqueue_begin(s));
     b.done_at.assign(nb, -1.0);
-    return enqueue_states(b);
+    BK_TRY(enqueue_states(b));
+    b.t_set_up = now_s();
+    return CG_OK;
 }
 
 // Reads the states behind the last cycle of the bucket and records its event.
@@ -508,8 +511,8 @@ int finish_bucket(const cg_system *sys, Bucket &b, cg_result *results) {
         r.cycles = h.cycles;
         r.rel_residual_estimate = h.est;
         r.rel_residual_true = h.true_res;
-        // latency: from the bucket's start (its set-up included) to the cycle
-        // boundary at which the host saw the system finish
+        // latency: the bucket's own set-up, and from the start of its wave's cycles to
+        // the cycle boundary at which the host saw the system finish
         r.seconds = (b.done_at[q] > 0.0 ? b.done_at[q] : t1) - b.t0;
         results[b.idx[q]] = r;
     }
@@ -528,8 +531,11 @@ struct Sweep {
     }
 };
 
-// Runs the buckets of a wave to their ends, each on its own stream.
+// Runs the buckets of a wave to their ends, each on its own stream.  No cycle starts
+// before all of them are set up; a bucket's time leaves that wait out.
 int run_wave(std::vector<std::unique_ptr<Bucket>> &wave, const cg_system *sys, const cg_opts &o, cg_result *results) {
+    const double t = now_s();
+    for (auto &b : wave) b->t0 += t - b->t_set_up;
     const int st = run_side_by_side(
         wave,
         [](Bucket &b, bool last, bool *go) -> int {

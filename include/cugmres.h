@@ -211,9 +211,12 @@ int cugmres_solve_batch(int device, int nsys, const cg_system *systems, const cg
  * max_bucket systems (0: as many as fit in half of the free device memory).
  * Every kernel of an Arnoldi step is one launch for the whole bucket; each
  * restart cycle of a bucket is one CUDA-graph replay; systems that stop early
- * skip the rest of their bucket's launches.  results[i].seconds is the time
- * from the start of system i's bucket (its operator set-up included) to the
- * cycle boundary at which it finished.  Supports CG_PREC_FP64 and CG_PREC_MIXED,
+ * skip the rest of their bucket's launches.  Up to eight buckets run side by
+ * side and share the GPU.  results[i].seconds is the operator set-up of system
+ * i's bucket plus the time from the first cycle to the cycle boundary at which
+ * it finished: without the other buckets' set-ups, but longer than alone by
+ * what they take of the GPU.  With a timeout, which counts that time, each
+ * bucket runs alone.  Supports CG_PREC_FP64 and CG_PREC_MIXED,
  * CG_ORTHO_DCGS2, no preconditioner, A x = b; other options return
  * CG_ERR_NOT_IMPLEMENTED.
  * Per-system convergence is in results[i].status. */

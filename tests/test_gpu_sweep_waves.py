@@ -42,3 +42,15 @@ def test_failing_bucket_ends_the_sweep(cuda_device):
         cg.solve_batch([systems[4], bad], device=cuda_device, restart=20, max_iter=60)
     _, infos = cg.solve_batch([systems[4], systems[0]], device=cuda_device, restart=20, max_iter=60, tol=1e-6)
     assert all(i["iterations"] > 0 for i in infos)
+
+
+def test_seconds_leave_out_the_set_ups_of_other_buckets(cuda_device):
+    """One step per system, so a bucket's time is its set-up.  The largest grid's, set up
+    first, used to hold the set-ups of the three buckets beside it as well: three times
+    its own.  The least of some runs, since allocations take a varying time."""
+    systems = [P.helmholtz(N, 2.0, seed=i, with_green=False) for N in (260, 200, 130, 96) for i in range(6)]
+    kw = dict(device=cuda_device, restart=20, max_iter=1, tol=1e-10)
+    cg.solve_batch(systems, **kw)  # tunes
+    alone = min(cg.solve_batch(systems[:6], **kw)[1][0]["seconds"] for _ in range(8))
+    beside = min(cg.solve_batch(systems, **kw)[1][0]["seconds"] for _ in range(8))
+    assert beside <= 1.8 * alone
