@@ -133,7 +133,13 @@ int ctx_op_view(const cg_ctx *c, OpView *v) {
 
 namespace {
 
-int cuerr(cudaError_t e) { return e == cudaSuccess ? CG_OK : (e == cudaErrorMemoryAllocation ? CG_ERR_OOM : CG_ERR_CUDA); }
+// The status is all that is left of an error: the runtime's own record of it would
+// be taken for a failure of the next kernel launch.
+int cuerr(cudaError_t e) {
+    if (e == cudaSuccess) return CG_OK;
+    cudaGetLastError();
+    return e == cudaErrorMemoryAllocation ? CG_ERR_OOM : CG_ERR_CUDA;
+}
 
 #define CG_TRY(expr)                  \
     do {                              \
@@ -277,7 +283,6 @@ int alloc_operator(cg_ctx *c) {
     if (!(c->shared_gpu && c->oparena && total <= c->oparena_cap)) {
         free_operator(c);
         if (int e = cuerr(cudaMalloc(&c->oparena, total))) {
-            cudaGetLastError();
             c->oparena = nullptr;
             return e;
         }
@@ -995,7 +1000,6 @@ static int set_operator_any(cg_ctx *c, int N, const cg_c128 *g_block, int kind, 
     if (bytes > c->scratch_cap) {
         free_scratch(c);
         if (int e = cuerr(cudaMalloc(&c->scratch, bytes))) {
-            cudaGetLastError();
             c->scratch = nullptr;
             return e;
         }

@@ -186,7 +186,12 @@ struct BucketBufs {
     }
 };
 
-int cu(cudaError_t e) { return e == cudaSuccess ? CG_OK : (e == cudaErrorMemoryAllocation ? CG_ERR_OOM : CG_ERR_CUDA); }
+// (as in cg_api.cu: no error is left for the next launch check to find)
+int cu(cudaError_t e) {
+    if (e == cudaSuccess) return CG_OK;
+    cudaGetLastError();
+    return e == cudaErrorMemoryAllocation ? CG_ERR_OOM : CG_ERR_CUDA;
+}
 #define BK_TRY(expr)                \
     do {                            \
         int _s = (expr);            \
@@ -634,7 +639,6 @@ extern "C" int cugmres_solve_buckets(int device, int nsys, const cg_system *sys,
             next_states += bucket.size();
             int st = setup_bucket(ctx, sys, o, *b);
             if (st == CG_ERR_OOM && !wave.empty()) {  // the wave's buffers stand in its way: alone
-                cudaGetLastError();
                 BK_TRY(run_wave(wave, sys, o, results));
                 wave_bytes = 0;
                 DevState *const states = b->bb.st_host;
