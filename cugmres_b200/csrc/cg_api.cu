@@ -267,6 +267,18 @@ void free_scratch(cg_ctx *c) {
     c->scratch_cap = 0;
 }
 
+// cudaMalloc that gives the kept temporaries back where they stand in its way, so
+// that keeping them takes no solve its memory
+int ctx_malloc(cg_ctx *c, void **p, size_t bytes) {
+    int e = cuerr(cudaMalloc(p, bytes));
+    if (e == CG_ERR_OOM && c->scratch) {
+        free_scratch(c);
+        e = cuerr(cudaMalloc(p, bytes));
+    }
+    if (e != CG_OK) *p = nullptr;
+    return e;
+}
+
 // lays the operator's arrays out for c->N and c->L; a context of a sweep, which
 // takes its systems largest grid first, keeps an allocation that is large enough
 int alloc_operator(cg_ctx *c) {
@@ -282,10 +294,7 @@ int alloc_operator(cg_ctx *c) {
     for (size_t b : bytes) total += (b + 255) & ~(size_t)255;
     if (!(c->shared_gpu && c->oparena && total <= c->oparena_cap)) {
         free_operator(c);
-        if (int e = cuerr(cudaMalloc(&c->oparena, total))) {
-            c->oparena = nullptr;
-            return e;
-        }
+        CG_TRY(ctx_malloc(c, &c->oparena, total));
         c->oparena_cap = total;
     }
     char *at = (char *)c->oparena;
@@ -793,6 +802,12 @@ bool all_finite(const double *p, size_t n) {
 }  // namespace
 
 // ================================================================== C-ABI
+namespace cg {
+void ctx_give_back(cg_ctx *c) {
+    if (c) free_scratch(c);
+}
+}  // namespace cg
+
 extern "C" {
 
 const char *cugmres_strerror(int s) {
@@ -1164,7 +1179,12 @@ int cugmres_solve(cg_ctx *c, const cg_c128 *b, cg_c128 *x, const cg_opts *opts_i
     const long long n = (long long)c->N * c->N;
     const size_t bytes = sizeof(double2) * n;
     const size_t esz = prec == 0 ? sizeof(double2) : sizeof(float2);
-    CG_TRY(ensure_krylov(c, m, std::max(1, o.max_iter), esz, S));
+    int room = ensure_krylov(c, m, std::max(1, o.max_iter), esz, S);
+    if (room == CG_ERR_OOM && c->scratch) {
+        free_scratch(c);
+        room = ensure_krylov(c, m, std::max(1, o.max_iter), esz, S);
+    }
+    CG_TRY(room);
     cudaStream_t s = c->stream;
     if (learned) {
         // flexible GMRES keeps z_j = M(v_j) next to the basis
@@ -1172,7 +1192,7 @@ int cugmres_solve(cg_ctx *c, const cg_c128 *b, cg_c128 *x, const cg_opts *opts_i
         if (c->zcap_bytes < zb) {
             dfree(c->Z);
             c->zcap_bytes = 0;
-            CG_CU(cudaMalloc(&c->Z, zb));
+            CG_TRY(ctx_malloc(c, &c->Z, zb));
             c->zcap_bytes = zb;
         }
         CG_TRY(fno::prepare(c->net, c->N, (float)c->k0h));
@@ -1203,7 +1223,7 @@ int cugmres_solve(cg_ctx *c, const cg_c128 *b, cg_c128 *x, const cg_opts *opts_i
         if (c->probe_cap_bytes < bytes) {
             dfree_t(c->probe_x);
             c->probe_cap_bytes = 0;
-            CG_CU(cudaMalloc((void **)&c->probe_x, bytes));
+            CG_TRY(ctx_malloc(c, (void **)&c->probe_x, bytes));
             c->probe_cap_bytes = bytes;
         }
         cg_opts po = o;

@@ -235,7 +235,7 @@ struct Bucket {
 };
 
 // Grids of the passes and the layout of the bucket's one allocation.
-int layout_bucket(Bucket &b, const cg_opts &o, int N, int nb) {
+int layout_bucket(cg_ctx *ctx, Bucket &b, const cg_opts &o, int N, int nb) {
     const int prec = o.precision == CG_PREC_MIXED ? 1 : 0;
     const int m = o.restart, L = b.ov.L;
     const long long n = (long long)N * N;
@@ -267,7 +267,12 @@ int layout_bucket(Bucket &b, const cg_opts &o, int N, int nb) {
     };
     size_t total = 0;
     for (const auto &e : a) total += al256(e.bytes);
-    BK_CU(cudaMalloc(&bb.all, total));
+    int st = cu(cudaMalloc(&bb.all, total));
+    if (st == CG_ERR_OOM) {  // the set-up's kept temporaries may stand in its way
+        ctx_give_back(ctx);
+        st = cu(cudaMalloc(&bb.all, total));
+    }
+    BK_TRY(st);
     char *at = (char *)bb.all;
     for (const auto &e : a) {
         *e.p = at;
@@ -301,7 +306,7 @@ int setup_bucket(cg_ctx *ctx, const cg_system *sys, const cg_opts &o, Bucket &b)
         BK_TRY(ctx_op_view(ctx, &ov));
         if (q == 0) {
             b.ov = ov;
-            BK_TRY(layout_bucket(b, o, N, nb));
+            BK_TRY(layout_bucket(ctx, b, o, N, nb));
             gq_elems = b.gq_elems;
             // (the context's own twiddles change with the next bucket's grid side)
             BK_CU(cudaMemcpyAsync(bb.TW, ov.tw64, sizeof(double2) * ov.ntw, cudaMemcpyDeviceToDevice, ov.stream));

@@ -173,6 +173,8 @@ int matvec_variant_persistent(int v);
 // marks a context whose GPU is shared with other contexts' solves (set by the
 // batch solver before its first operator)
 void ctx_set_shared_gpu(cg_ctx *c, bool on);
+// frees what a context of a sweep keeps of one operator's set-up for the next
+void ctx_give_back(cg_ctx *c);
 // Device buffers of a context's current operator (FP64), read by the bucket
 // solver, which copies each system's spectrum and contrast into its own arrays.
 struct OpView {

@@ -46,3 +46,25 @@ def test_sweep_goes_on_after_a_system_that_does_not_fit(little_memory):
     assert e.value.status == cg._lib.CG_ERR_OOM
     _, infos = cg.solve_batch([small], restart=8, max_iter=3)
     assert infos[0]["iterations"] == 3
+
+
+# an operator's arrays in a context: spectra, contrasts, T, three vectors, twiddles
+OPERATOR = 24 * (L // 2 + 1) ** 2 + 16 * N * N + 16 * N * L + 3 * UNIT + 24 * 4 * L
+SLACK = 48 * 10 ** 6  # workspaces and what the driver takes; the set-up's temporaries are 92 MB
+
+
+def test_sweep_has_the_memory_of_its_set_up(little_memory):
+    """A bucket that fits beside the operator's arrays, but not beside the temporaries of their set-up."""
+    pr = problems.helmholtz(N, 2.0, seed=0, with_green=False)
+    bucket = 16 * N * L + 16 * (L // 2 + 1) ** 2 + 8 * N * N + 2 * UNIT
+    restart = (little_memory - OPERATOR - bucket - SLACK) // UNIT - 2
+    _, infos = cg.solve_batch([pr], restart=int(restart), max_iter=3)
+    assert infos[0]["iterations"] == 3
+
+
+def test_contexts_have_the_memory_of_their_set_up(little_memory):
+    big = problems.helmholtz(N, 2.0, seed=0, with_green=False)
+    small = problems.helmholtz(16, 2.0, seed=0, with_green=False)
+    restart = (little_memory - OPERATOR - SLACK) // UNIT - 2
+    _, infos = cg.solve_batch([big, small], mode="contexts", workers=2, restart=int(restart), max_iter=3)
+    assert [i["iterations"] for i in infos] == [3, 3]
