@@ -513,9 +513,14 @@ cudaLaunchConfig_t cluster_config(int nsys, int bytes, cudaLaunchAttribute *at, 
     cfg.numAttrs = 1;
     return cfg;
 }
-template <typename K> int cluster_optin(K kern, int bytes) {
-    if (int e = smem_optin(kern, bytes)) return e;
-    return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+// 220 KB: a CTA's shared memory (227 KB) less these kernels' static arrays.  Always
+// the same limit, whatever the launch needs (see smem_optin, whose look at the
+// kernel would add 0.4 us to the 26 of a product that is waited for).
+constexpr int SC_SMEM = 220 * 1024;
+template <typename K> int cluster_optin(K kern) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SC_SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    return (int)e;
 }
 
 template <typename C, int NP>
@@ -523,7 +528,7 @@ int launch(void *V, long long n, const KrylovPtrs &kp, int m, const MatvecArgs &
     typedef typename real_of<C>::type R;
     auto kern = k_small_cycle<C, NP>;
     const int bytes = small_smem<C, NP>(a.N, m).bytes;
-    if (int e = cluster_optin(kern, bytes)) return e;
+    if (int e = cluster_optin(kern)) return e;
     cudaLaunchAttribute at;
     const cudaLaunchConfig_t cfg = cluster_config(kp.nsys, bytes, &at, s);
     return (int)cudaLaunchKernelEx(&cfg, kern, (C *)V, n, kp, a.N, (const R *)a.cdiag, (const C *)a.gq,
@@ -533,22 +538,20 @@ template <typename C, int NP> int launch_mv(const void *x, void *y, const Matvec
     typedef typename real_of<C>::type R;
     auto kern = k_small_matvec<C, NP>;
     const int bytes = small_smem<C, NP>(a.N, 0).bytes;
-    if (int e = cluster_optin(kern, bytes)) return e;
+    if (int e = cluster_optin(kern)) return e;
     cudaLaunchAttribute at;
     const cudaLaunchConfig_t cfg = cluster_config(1, bytes, &at, s);
     return (int)cudaLaunchKernelEx(&cfg, kern, (const C *)x, (C *)y, a.N, (const R *)a.cdiag, (const C *)a.gq,
                                    (const C *)a.tw, a.transpose);
 }
 
-// 220 KB: a CTA's shared memory (227 KB) less this kernel's static arrays
-constexpr int SC_SMEM = 220 * 1024;
 template <typename C, int NP> bool fits(int N, int m) {
     static const int most = [] {  // clusters that the device holds at that size
         auto kern = k_small_cycle<C, NP>;
         cudaLaunchAttribute at;
         const cudaLaunchConfig_t cfg = cluster_config(1, SC_SMEM, &at, nullptr);
         int c = 0;
-        if (cluster_optin(kern, SC_SMEM) != 0 || cudaOccupancyMaxActiveClusters(&c, kern, &cfg) != cudaSuccess) {
+        if (cluster_optin(kern) != 0 || cudaOccupancyMaxActiveClusters(&c, kern, &cfg) != cudaSuccess) {
             cudaGetLastError();
             c = 0;
         }
