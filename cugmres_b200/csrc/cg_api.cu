@@ -1560,16 +1560,14 @@ int cugmres_solve(cg_ctx *c, const cg_c128 *b, cg_c128 *x, const cg_opts *opts_i
                     &slot->exec));
             } else {
                 cudaGraph_t g = nullptr;
-                CG_CU(cudaStreamBeginCapture(c->cap_stream, cudaStreamCaptureModeThreadLocal));
-                int e1 = ss_on ? enqueue_cycle_ss(c->cap_stream, 0, ss_nblk, true) : enqueue_cycle(1, c->cap_stream);
-                int e2 = e1 == CG_OK ? enqueue_begin(c->cap_stream) : e1;
-                cudaError_t ce = cudaStreamEndCapture(c->cap_stream, &g);
-                if (e2 != CG_OK || ce != cudaSuccess) {
-                    if (g) cudaGraphDestroy(g);
-                    cudaGetLastError();
-                    return e2 != CG_OK ? e2 : CG_ERR_CUDA;
-                }
-                ce = cudaGraphInstantiate(&slot->exec, g, 0);
+                CG_TRY(capture_graph(
+                    c->cap_stream,
+                    [&](cudaStream_t q) -> int {
+                        CG_TRY(ss_on ? enqueue_cycle_ss(q, 0, ss_nblk, true) : enqueue_cycle(1, q));
+                        return enqueue_begin(q);
+                    },
+                    &g));
+                const cudaError_t ce = cudaGraphInstantiate(&slot->exec, g, 0);
                 cudaGraphDestroy(g);
                 if (ce != cudaSuccess) {
                     slot->exec = nullptr;

@@ -212,8 +212,10 @@ int axpy2_blocks(int prec_v, int sms, int mcap, long long n);
 __host__ __device__ inline int dots2_part_ld(int mcap) { return 2 * (mcap + 1) > 64 ? 2 * (mcap + 1) : 64; }
 int launch_backsolve(const KrylovPtrs &kp, cudaStream_t s);
 int launch_cycle_begin(const KrylovPtrs &kp, int nparts, cudaStream_t s);
-// sets a graph loop's condition: some system of kp has not stopped
-int launch_loop_test(const KrylovPtrs &kp, cudaGraphConditionalHandle h, cudaStream_t s);
+// adds the kernel that sets a graph loop's condition (some system of kp has not
+// stopped) to the loop's body `in`, behind node `after`
+int add_loop_test(const KrylovPtrs &kp, cudaGraphConditionalHandle h, cudaGraph_t in, cudaGraphNode_t after,
+                  cudaGraphNode_t *node);
 // ortho 0: delayed CGS2, 1: CGS2, for the cycle k_cycle_begin has just set up
 int launch_set_ortho(const KrylovPtrs &kp, int ortho, cudaStream_t s);
 // Whole delayed-CGS2 cycles of small grids in one kernel (cg_small.cu): 1 where
@@ -265,47 +267,63 @@ int launch_norm2(int prec, const void *v, long long n, double *npart, unsigned i
                  cudaStream_t s);
 int launch_convert(int from_prec, int to_prec, const void *src, void *dst, long long n, cudaStream_t s);
 
+// One stream capture of what `enqueue` (returning a CG_* status) launches on `cap`.
+template <typename E> int capture_graph(cudaStream_t cap, E enqueue, cudaGraph_t *out) {
+    *out = nullptr;
+    if (cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+        cudaGetLastError();
+        return 2;  // CG_ERR_CUDA
+    }
+    const int e = enqueue(cap);
+    const cudaError_t ce = cudaStreamEndCapture(cap, out);
+    if (e == 0 && ce == cudaSuccess) return 0;
+    if (*out) cudaGraphDestroy(*out);
+    *out = nullptr;
+    cudaGetLastError();
+    return e != 0 ? e : 2;
+}
+
 // A restart cycle as a CUDA graph: [while some system runs: `body`] -> `tail`,
-// both captured on `cap` by the callbacks (which return a CG_* status).  The
+// both captured on `cap` from the callbacks (which return a CG_* status).  The
 // loop is a conditional node whose last kernel looks at the systems' stop flags,
 // so the graph holds the steps of one body whatever the restart length: it is
 // captured and instantiated in the time of a few launches, and a cycle that
 // converges early does not run through the launches of the steps it did not
 // take (64^2, restart 500, 55 steps: 2670 of 3000 launches returned at once).
+// Body and tail are captured apart and join as child graphs once both are whole, so
+// that a capture that fails is dropped before the loop exists (a process whose
+// launches were refused during captures straight into the body crashed).
 template <typename B, typename T>
 int cycle_graph(const KrylovPtrs &kp, cudaStream_t cap, B body, T tail, cudaGraphExec_t *out) {
-    cudaGraph_t g = nullptr;
-    if (cudaGraphCreate(&g, 0) != cudaSuccess) return 2;  // CG_ERR_CUDA
-    cudaGraphConditionalHandle h;
-    cudaGraphNodeParams np = {};
-    np.type = cudaGraphNodeTypeConditional;
-    cudaGraphNode_t node = nullptr;
-    int st = 2;
-    if (cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault) == cudaSuccess) {
+    *out = nullptr;
+    cudaGraph_t gb = nullptr, gt = nullptr, g = nullptr;
+    int st = capture_graph(cap, body, &gb);
+    if (st == 0) st = capture_graph(cap, tail, &gt);
+    auto build = [&]() -> int {
+        cudaGraphConditionalHandle h;
+        cudaGraphNodeParams np = {};
+        np.type = cudaGraphNodeTypeConditional;
+        cudaGraphNode_t loop, steps, test, rest;
+        if (cudaGraphCreate(&g, 0) != cudaSuccess ||
+            cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault) != cudaSuccess)
+            return 2;
         np.conditional.handle = h;
         np.conditional.type = cudaGraphCondTypeWhile;
         np.conditional.size = 1;
-        if (cudaGraphAddNode(&node, g, nullptr, 0, &np) == cudaSuccess) st = 0;
-    }
-    auto capture = [&](cudaGraph_t into, const cudaGraphNode_t *dep, size_t ndep, auto &&enqueue) -> int {
-        if (cudaStreamBeginCaptureToGraph(cap, into, dep, nullptr, ndep, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
+        if (cudaGraphAddNode(&loop, g, nullptr, 0, &np) != cudaSuccess) return 2;
+        const cudaGraph_t in = np.conditional.phGraph_out[0];
+        if (cudaGraphAddChildGraphNode(&steps, in, nullptr, 0, gb) != cudaSuccess ||
+            add_loop_test(kp, h, in, steps, &test) != 0 ||
+            cudaGraphAddChildGraphNode(&rest, g, &loop, 1, gt) != cudaSuccess ||
+            cudaGraphInstantiate(out, g, 0) != cudaSuccess) {
+            *out = nullptr;
             return 2;
-        const int e = enqueue();
-        cudaGraph_t same = nullptr;
-        const cudaError_t ce = cudaStreamEndCapture(cap, &same);
-        return e != 0 ? e : ce != cudaSuccess ? 2 : 0;
+        }
+        return 0;
     };
-    if (st == 0)
-        st = capture(np.conditional.phGraph_out[0], nullptr, 0, [&]() -> int {
-            const int e = body(cap);
-            return e != 0 ? e : launch_loop_test(kp, h, cap) != 0 ? 2 : 0;
-        });
-    if (st == 0) st = capture(g, &node, 1, [&]() -> int { return tail(cap); });
-    if (st == 0 && cudaGraphInstantiate(out, g, 0) != cudaSuccess) {
-        *out = nullptr;
-        st = 2;
-    }
-    cudaGraphDestroy(g);
+    if (st == 0) st = build();
+    for (cudaGraph_t q : {g, gt, gb})
+        if (q) cudaGraphDestroy(q);
     if (st != 0) cudaGetLastError();
     return st;
 }

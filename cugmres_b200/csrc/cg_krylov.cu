@@ -505,9 +505,16 @@ __global__ void k_loop_test(KrylovPtrs kp, cudaGraphConditionalHandle h) {
     if (threadIdx.x == 0) cudaGraphSetConditional(h, run ? 1u : 0u);
 }
 
-int launch_loop_test(const KrylovPtrs &kp, cudaGraphConditionalHandle h, cudaStream_t s) {
-    k_loop_test<<<1, 32, 0, s>>>(kp, h);
-    return (int)cudaGetLastError();
+int add_loop_test(const KrylovPtrs &kp, cudaGraphConditionalHandle h, cudaGraph_t in, cudaGraphNode_t after,
+                  cudaGraphNode_t *node) {
+    KrylovPtrs k = kp;
+    void *args[] = {&k, &h};
+    cudaKernelNodeParams p = {};
+    p.func = (void *)k_loop_test;
+    p.gridDim = dim3(1);
+    p.blockDim = dim3(32);
+    p.kernelParams = args;
+    return (int)cudaGraphAddKernelNode(node, in, &after, 1, &p);
 }
 
 int launch_norm2(int prec, const void *v, long long n, double *npart, unsigned int *counter, double *out, int nblk,
