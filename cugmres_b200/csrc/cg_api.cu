@@ -108,7 +108,7 @@ struct cg_ctx {
 namespace cg {
 // entries of the twiddle tables: 4 L of cg_fft.cuh, then those of cg_wfft.cuh,
 // which the embedding of the one-kernel cycles uses
-static size_t tw_entries(int L) { return 4 * (size_t)L + (L == 128 ? wtw_entries(wplan_r1(L / 2)) : 0); }
+static size_t tw_entries(int L) { return 4 * (size_t)L + (L == WPlan::L ? WTW_ENTRIES : 0); }
 void ctx_set_shared_gpu(cg_ctx *c, bool on) {
     if (c) c->shared_gpu = on;
 }
@@ -1002,7 +1002,7 @@ static int set_operator_any(cg_ctx *c, int N, const cg_c128 *g_block, int kind, 
         }
     }
     for (size_t i = 4 * (size_t)L; i < ntw; i++) {
-        const double a = 2.0 * pi * (double)wtw_exponent(L, wplan_r1(L / 2), (int)(i - 4 * (size_t)L)) / (double)L;
+        const double a = 2.0 * pi * (double)wtw_exponent((int)(i - 4 * (size_t)L)) / (double)L;
         tw[i] = make_double2(cos(a), -sin(a));
     }
     for (size_t i = 0; i < tw.size(); i++) twf[i] = make_float2((float)tw[i].x, (float)tw[i].y);

@@ -41,13 +41,14 @@ namespace {
 namespace cgr = cooperative_groups;
 
 constexpr int SC_CTAS = 16, SC_THREADS = 256, SC_WARPS = SC_THREADS / 32;
+constexpr int NP = WPlan::NP;
 
 // Shared memory of one CTA, in bytes from the start.
 struct SmallSmem {
     int su, sw, sc, tb, rb, ex, part, d1, d2, tv, cs, sn, col, pc, bytes;
 };
-template <typename C, int NP> __host__ __device__ constexpr SmallSmem small_smem(int N, int m) {
-    typedef WPlan<NP> P;
+template <typename C> __host__ __device__ constexpr SmallSmem small_smem(int N, int m) {
+    typedef WPlan P;
     const int rpc = (N + SC_CTAS - 1) / SC_CTAS, ns = rpc * N, e = sizeof(C);
     SmallSmem s{};
     int o = 0;
@@ -111,9 +112,9 @@ template <typename C> __device__ __forceinline__ void dot2(C a, C u, C w, double
 }
 
 // One CTA's share of the operator: the arrays, and this lane's place in them.
-template <typename C, int NP> struct SmallOp {
+template <typename C> struct SmallOp {
     typedef typename real_of<C>::type R;
-    typedef WPlan<NP> P;
+    typedef WPlan P;
     static constexpr int E = P::E, LPT = P::LPT, TPW = P::TPW, CPC = 2 * NP / SC_CTAS;
     static_assert(TPW == 4 && CPC % TPW == 0 && CPC / TPW * 2 <= SC_WARPS, "a warp pair per four columns");
     C *su, *sw, *tb, *rb, *mine;
@@ -165,7 +166,7 @@ template <typename C, int NP> struct SmallOp {
                 reg[i] = czero<C>();
                 if (rl < rows && x < N) reg[i] = transpose ? su[rl * N + x] : cscale(su[rl * N + x], sc[rl * N + x]);
             }
-            wfft<NP, false>(reg, mine, twl, t, u4, p);
+            wfft<false>(reg, mine, twl, t, u4, p);
             if (rl < rows) {
 #pragma unroll
                 for (int i = 0; i < E; i++) {
@@ -183,11 +184,11 @@ template <typename C, int NP> struct SmallOp {
                 const int y = t + i * LPT;
                 reg[i] = y < N ? tb[c_loc * ldt + y] : czero<C>();
             }
-            wfft<NP, false>(reg, mine, twl, t, u4, p);
+            wfft<false>(reg, mine, twl, t, u4, p);
 #pragma unroll
             for (int i = 0; i < E; i++) reg[i] = cmul(reg[i], gv[i]);
             __syncwarp();
-            wfft<NP, true>(reg, mine, twl, t, u4, p);
+            wfft<true>(reg, mine, twl, t, u4, p);
             auto put = [&](int i, C v) {
                 const int y = t + i * LPT;
                 if (y < N) cl.map_shared_rank(rb, y / rpc)[(y % rpc) * ldr + rank * CPC + c_loc] = v;
@@ -201,7 +202,7 @@ template <typename C, int NP> struct SmallOp {
             C reg[E];
 #pragma unroll
             for (int i = 0; i < E; i++) reg[i] = rl < rows ? rb[rl * ldr + p * NP + t + i * LPT] : czero<C>();
-            wfft<NP, true>(reg, mine, twl, t, u4, p);
+            wfft<true>(reg, mine, twl, t, u4, p);
             auto put = [&](int i, C v) {
                 const int x = t + i * LPT;
                 if (rl < rows && x < N) {
@@ -216,7 +217,7 @@ template <typename C, int NP> struct SmallOp {
     }
 };
 
-template <typename C, int NP>
+template <typename C>
 __global__ void __launch_bounds__(SC_THREADS, 1)
 k_small_cycle(C *V, long long n, KrylovPtrs kp, int N, const typename real_of<C>::type *cdiag, const C *gq,
               const C *__restrict__ tw, int transpose, int m, long long sys_c, long long sys_gq) {
@@ -230,7 +231,7 @@ k_small_cycle(C *V, long long n, KrylovPtrs kp, int N, const typename real_of<C>
     cgr::cluster_group cl = cgr::this_cluster();
     const int rank = (int)cl.block_rank();
     extern __shared__ __align__(16) unsigned char smem[];
-    const SmallSmem lay = small_smem<C, NP>(N, m);
+    const SmallSmem lay = small_smem<C>(N, m);
     double *part = reinterpret_cast<double *>(smem + lay.part);
     double2 *D1 = reinterpret_cast<double2 *>(smem + lay.d1), *D2 = reinterpret_cast<double2 *>(smem + lay.d2);
     double2 *tvs = reinterpret_cast<double2 *>(smem + lay.tv), *css = reinterpret_cast<double2 *>(smem + lay.cs);
@@ -245,7 +246,7 @@ k_small_cycle(C *V, long long n, KrylovPtrs kp, int N, const typename real_of<C>
     __shared__ int fin_stop;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    SmallOp<C, NP> op(smem, lay, N, rank, gq, tw, transpose);
+    SmallOp<C> op(smem, lay, N, rank, gq, tw, transpose);
     C *su = op.su, *sw = op.sw;
     const int ns = op.ns;
     const size_t base = (size_t)op.r0 * N;
@@ -481,13 +482,13 @@ k_small_cycle(C *V, long long n, KrylovPtrs kp, int N, const typename real_of<C>
 }
 
 // y = A x (A^T x) as one launch.
-template <typename C, int NP>
+template <typename C>
 __global__ void __launch_bounds__(SC_THREADS, 1)
 k_small_matvec(const C *x, C *y, int N, const typename real_of<C>::type *cdiag, const C *gq, const C *__restrict__ tw,
                int transpose) {
     cgr::cluster_group cl = cgr::this_cluster();
     extern __shared__ __align__(16) unsigned char smem[];
-    SmallOp<C, NP> op(smem, small_smem<C, NP>(N, 0), N, (int)cl.block_rank(), gq, tw, transpose);
+    SmallOp<C> op(smem, small_smem<C>(N, 0), N, (int)cl.block_rank(), gq, tw, transpose);
     const size_t base = (size_t)op.r0 * N;
     for (int e = threadIdx.x; e < op.ns; e += SC_THREADS) {
         op.su[e] = x[base + e];
@@ -523,21 +524,21 @@ template <typename K> int cluster_optin(K kern) {
     return (int)e;
 }
 
-template <typename C, int NP>
+template <typename C>
 int launch(void *V, long long n, const KrylovPtrs &kp, int m, const MatvecArgs &a, cudaStream_t s) {
     typedef typename real_of<C>::type R;
-    auto kern = k_small_cycle<C, NP>;
-    const int bytes = small_smem<C, NP>(a.N, m).bytes;
+    auto kern = k_small_cycle<C>;
+    const int bytes = small_smem<C>(a.N, m).bytes;
     if (int e = cluster_optin(kern)) return e;
     cudaLaunchAttribute at;
     const cudaLaunchConfig_t cfg = cluster_config(kp.nsys, bytes, &at, s);
     return (int)cudaLaunchKernelEx(&cfg, kern, (C *)V, n, kp, a.N, (const R *)a.cdiag, (const C *)a.gq,
                                    (const C *)a.tw, a.transpose, m, a.sys_c, a.sys_gq);
 }
-template <typename C, int NP> int launch_mv(const void *x, void *y, const MatvecArgs &a, cudaStream_t s) {
+template <typename C> int launch_mv(const void *x, void *y, const MatvecArgs &a, cudaStream_t s) {
     typedef typename real_of<C>::type R;
-    auto kern = k_small_matvec<C, NP>;
-    const int bytes = small_smem<C, NP>(a.N, 0).bytes;
+    auto kern = k_small_matvec<C>;
+    const int bytes = small_smem<C>(a.N, 0).bytes;
     if (int e = cluster_optin(kern)) return e;
     cudaLaunchAttribute at;
     const cudaLaunchConfig_t cfg = cluster_config(1, bytes, &at, s);
@@ -545,9 +546,9 @@ template <typename C, int NP> int launch_mv(const void *x, void *y, const Matvec
                                    (const C *)a.tw, a.transpose);
 }
 
-template <typename C, int NP> bool fits(int N, int m) {
+template <typename C> bool fits(int N, int m) {
     static const int most = [] {  // clusters that the device holds at that size
-        auto kern = k_small_cycle<C, NP>;
+        auto kern = k_small_cycle<C>;
         cudaLaunchAttribute at;
         const cudaLaunchConfig_t cfg = cluster_config(1, SC_SMEM, &at, nullptr);
         int c = 0;
@@ -557,7 +558,7 @@ template <typename C, int NP> bool fits(int N, int m) {
         }
         return c;
     }();
-    return most > 0 && small_smem<C, NP>(N, m).bytes <= SC_SMEM;
+    return most > 0 && small_smem<C>(N, m).bytes <= SC_SMEM;
 }
 
 }  // namespace
@@ -573,18 +574,18 @@ int small_cycle_fits(int prec, int N, int L, int m) {
         }
         return true;
     }();
-    if (!on || L != 128) return 0;
-    return prec == 0 ? fits<double2, 64>(N, m) : fits<float2, 64>(N, m);
+    if (!on || L != WPlan::L) return 0;
+    return prec == 0 ? fits<double2>(N, m) : fits<float2>(N, m);
 }
 
 int launch_small_cycle(int prec, void *V, long long n, const KrylovPtrs &kp, int m, const MatvecArgs &a, cudaStream_t s) {
-    if (a.L != 128 || m > kp.mcap) return (int)cudaErrorInvalidValue;
-    return prec == 0 ? launch<double2, 64>(V, n, kp, m, a, s) : launch<float2, 64>(V, n, kp, m, a, s);
+    if (a.L != WPlan::L || m > kp.mcap) return (int)cudaErrorInvalidValue;
+    return prec == 0 ? launch<double2>(V, n, kp, m, a, s) : launch<float2>(V, n, kp, m, a, s);
 }
 
 int launch_small_matvec(int prec, const void *x, void *y, const MatvecArgs &a, cudaStream_t s) {
-    if (a.L != 128) return (int)cudaErrorInvalidValue;
-    return prec == 0 ? launch_mv<double2, 64>(x, y, a, s) : launch_mv<float2, 64>(x, y, a, s);
+    if (a.L != WPlan::L) return (int)cudaErrorInvalidValue;
+    return prec == 0 ? launch_mv<double2>(x, y, a, s) : launch_mv<float2>(x, y, a, s);
 }
 
 }  // namespace cg
