@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(D2_THREADS, 2) k_dots2t(const CV *__restrict__
 // block accumulates it in a single shared-memory slot (chunks of cs vectors)
 // without atomics; block partials and the last-block sum as in k_dots2t.
 // MINB blocks per SM: 2 where the tiles outnumber the SMs (148 registers had kept
-// one 8-warp block, 32 KB of loads, on an SM: 512^2 FP64 at 3.4 TB/s).
+// one 8-warp block, 32 KB of loads, on an SM: 512^2 FP64 GMRES(100) at 4.0 TB/s, now 4.5).
 template <typename CV, int U, int MINB = 1>
 __global__ void __launch_bounds__(D2_THREADS, MINB) k_dots2s(const CV *__restrict__ V, long long n, KrylovPtrs kp) {
     kp = kp_sys(kp);  // this block's system of a bucket

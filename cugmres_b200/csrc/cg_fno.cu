@@ -864,8 +864,8 @@ k_proj_bwd(const __nv_bfloat16 *__restrict__ zq, const float *__restrict__ dout,
 // added to the sums by FP32 additions.  Error of dW against 64 bits, random values of
 // mean 1, relative rms, 16 x 64 x 64 / 16 x 160 x 160 cells, NO = 128: FP32 fused multiply-adds 2.8e-8 /
 // 3.5e-8, a chain of m16n8k16 2.5e-7 / 1.6e-6, this 2.7e-8 / 2.4e-8 (steps of 16 cells 3.0e-8 / 2.7e-8).
-// Time on 16 x 64 x 64 cells, launch included: 49 us (NO = 128) and 31 us (NO = 32) by FP32 fused
-// multiply-adds from shared memory, 10 and 9 by the chain, 13 and 10.5 by this.
+// Time on 16 x 64 x 64 cells (ncu): 73 us (NO = 128) and 45 us (NO = 32) by FP32 fused
+// multiply-adds from shared memory, 8 and 6 by the chain, 10 and 7 by this.
 constexpr int WG_CELLS = 64, WG_THREADS = 128;
 __device__ __forceinline__ uint32_t wg_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void wg_copy16(void *dst, const void *src, bool ok) {
@@ -1054,7 +1054,8 @@ k_lift_bwd(const float *__restrict__ dv0, const RT *__restrict__ r, const float 
 
 // dst[i] = sum_b part[b][i] (fixed order).  A block owns 32 outputs; its 32 warps
 // share the partial rows, so that a few hundred rows are a dozen loads deep: one
-// thread per output walked them in 35 us, whatever their size (now 3 to 5 us).
+// thread per output walked them in 36 us, whatever their size (now 7.5, launch latency
+// included; 16 x 64 x 64 cells).
 constexpr int REDUCE_ROWS = 32;
 __global__ void __launch_bounds__(32 * REDUCE_ROWS) k_reduce(const float *__restrict__ part, int nblk, int cnt,
                                                              float *__restrict__ dst) {

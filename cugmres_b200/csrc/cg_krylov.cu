@@ -287,8 +287,9 @@ __global__ void k_givens(KrylovPtrs kp) {
 // at a time from the last: the first warp solves the diagonal block from shared
 // memory, one unknown per lane handed round by shuffles, then every thread takes
 // the block's columns off its rows of the right-hand side with independent loads.
-// One warp walking the columns waited for each column's entries (41 us for 48
-// columns; now 33 for 100); the operations and their order per entry are the same.
+// One warp walking the columns waited for each column's entries (48 / 100 columns, ncu,
+// cold caches: 68 / 176 us, now 17 / 48); the operations and their order per entry are
+// the same.
 constexpr int BS_THREADS = 256;
 __global__ void __launch_bounds__(BS_THREADS) k_backsolve(KrylovPtrs kp) {
     kp = kp_sys(kp);  // this block's system of a bucket

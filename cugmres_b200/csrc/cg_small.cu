@@ -21,8 +21,9 @@
 // instead of all of them, which is the price: it ends the gain on larger grids.
 // Whole FP64 solves of up to 100 steps, us per step, launched / one kernel: 33^2
 // 32.2 / 15.9, 48^2 32.8 / 16.4, 64^2 33.8 / 17.5; the same kernel built for L = 256:
-// 65^2 31.1 / 26.5, 80^2 32.1 / 32.5, 96^2 32.8 / 35.5, 112^2 33.2 / 46, so only L = 128 (33 <=
-// N <= 64) is.  A bucket of systems runs one cluster per system.
+// 65^2 31.1 / 26.5, 80^2 32.1 / 32.5, 96^2 32.8 / 35.5, 112^2 33.2 / 46.  Only L = 128 (33 <=
+// N <= 64) is built; the sides from 65 to 79 that L = 256 would serve faster are launched.
+// A bucket of systems runs one cluster per system.
 //
 // Transforms: cg_wfft.cuh, NP = L / 2 = 64, four per warp; a pair of warps takes
 // the two parities of four lines.
