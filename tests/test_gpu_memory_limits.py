@@ -50,7 +50,7 @@ def test_sweep_goes_on_after_a_system_that_does_not_fit(little_memory):
 
 # an operator's arrays in a context: spectra, contrasts, T, three vectors, twiddles
 OPERATOR = 24 * (L // 2 + 1) ** 2 + 16 * N * N + 16 * N * L + 3 * UNIT + 24 * 4 * L
-SLACK = 48 * 10 ** 6  # workspaces and what the driver takes; the set-up's temporaries are 92 MB
+SLACK = 48 * 10 ** 6  # workspaces and what the runtime takes; the set-up's temporaries are 92 MB
 
 
 def test_sweep_has_the_memory_of_its_set_up(little_memory):

@@ -54,3 +54,28 @@ def test_seconds_leave_out_the_set_ups_of_other_buckets(cuda_device):
     alone = min(cg.solve_batch(systems[:6], **kw)[1][0]["seconds"] for _ in range(8))
     beside = min(cg.solve_batch(systems, **kw)[1][0]["seconds"] for _ in range(8))
     assert beside <= 1.8 * alone
+
+
+def test_time_limit_ends_each_bucket(cuda_device):
+    """With a time limit the buckets run one after the other, each against its own clock: the
+    limit ends the hard systems at a cycle boundary and leaves the easy one alone."""
+    import ctypes
+    lib = cg._lib
+    systems = [P.helmholtz(256, 12.0, seed=1, with_green=False), P.helmholtz(200, 12.0, seed=2, with_green=False),
+               P.helmholtz(40, 1.5, seed=3, with_green=False)]
+    cg.solve_batch(systems, device=cuda_device, restart=20, max_iter=20)  # tunes
+    arr, keep = (lib.CgSystem * 3)(), []
+    for i, s in enumerate(systems):
+        chi, b = np.ascontiguousarray(s["chi"]), np.ascontiguousarray(s["b"], np.complex128)
+        x = np.zeros_like(b)
+        keep.append((chi, b, x))
+        arr[i] = lib.CgSystem(s["N"], None, chi.ctypes.data, s["chi_scale"], b.ctypes.data, x.ctypes.data, s["k0"], s["h"])
+    o = lib.CgOpts()
+    lib.lib().cugmres_default_opts(ctypes.byref(o))
+    o.restart, o.max_iter, o.tol, o.timeout_s = 20, 10 ** 6, 1e-10, 1.0
+    res = (lib.CgResult * 3)()
+    lib.check(lib.lib().cugmres_solve_buckets(cuda_device, 3, arr, ctypes.byref(o), 0, res), "solve_buckets")
+    assert [r.status for r in res] == [lib.CG_ERR_TIMEOUT, lib.CG_ERR_TIMEOUT, lib.CG_OK]
+    for r in list(res)[:2]:
+        assert 1.0 < r.seconds < 3.0 and r.iterations > 100
+    assert res[2].rel_residual_true <= 1e-10
