@@ -58,7 +58,8 @@ def test_seconds_leave_out_the_set_ups_of_other_buckets(cuda_device):
 
 def test_time_limit_ends_each_bucket(cuda_device):
     """With a time limit the buckets run one after the other, each against its own clock: the
-    limit ends the hard systems at a cycle boundary and leaves the easy one alone."""
+    limit ends the hard systems at a cycle boundary and leaves the easy one alone.  (The
+    limit counts a bucket's set-up, whose allocations have been seen to take a second.)"""
     import ctypes
     lib = cg._lib
     systems = [P.helmholtz(256, 12.0, seed=1, with_green=False), P.helmholtz(200, 12.0, seed=2, with_green=False),
@@ -72,10 +73,10 @@ def test_time_limit_ends_each_bucket(cuda_device):
         arr[i] = lib.CgSystem(s["N"], None, chi.ctypes.data, s["chi_scale"], b.ctypes.data, x.ctypes.data, s["k0"], s["h"])
     o = lib.CgOpts()
     lib.lib().cugmres_default_opts(ctypes.byref(o))
-    o.restart, o.max_iter, o.tol, o.timeout_s = 20, 10 ** 6, 1e-10, 1.0
+    o.restart, o.max_iter, o.tol, o.timeout_s = 20, 10 ** 6, 1e-10, 2.5
     res = (lib.CgResult * 3)()
     lib.check(lib.lib().cugmres_solve_buckets(cuda_device, 3, arr, ctypes.byref(o), 0, res), "solve_buckets")
     assert [r.status for r in res] == [lib.CG_ERR_TIMEOUT, lib.CG_ERR_TIMEOUT, lib.CG_OK]
     for r in list(res)[:2]:
-        assert 1.0 < r.seconds < 3.0 and r.iterations > 100
+        assert 2.5 < r.seconds < 6.0 and r.iterations > 100
     assert res[2].rel_residual_true <= 1e-10
